@@ -26,8 +26,33 @@ template <typename T> using cplx = typename cplx_t<T>::type;
 template <typename V> __device__ __forceinline__ V cmk(decltype(V().x) x, decltype(V().x) y) {
     V r; r.x = x; r.y = y; return r;
 }
+#ifdef RK_PACKED_F32
+// complex64 sums and differences as one packed instruction (add / sub.rn.f32x2, sm_100;
+// each half rounds as the scalar instruction does): the butterflies are mostly these.
+// Only the lean passes take them (rk_lean.cuh: contiguous 1024-point lines 45.3 -> 43.9
+// us, strided 256-point lines 51.3 -> 49.0): the register pairs they need made the general
+// kernels slower where those are short of registers (1000 x 3001 Bluestein 85.7 -> 88.1
+// us, the 256 x 256 plane pass 97 -> 100 us).
+__device__ __forceinline__ unsigned long long f2_bits(float2 a) {
+    return ((unsigned long long)__float_as_uint(a.y) << 32) | __float_as_uint(a.x);
+}
+__device__ __forceinline__ float2 f2_from_bits(unsigned long long u) {
+    return make_float2(__uint_as_float((unsigned)u), __uint_as_float((unsigned)(u >> 32)));
+}
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from_bits(r);
+}
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from_bits(r);
+}
+#else
 __device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+#endif
 __device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -63,6 +64,8 @@ struct PairInfo {
     int nl_rows, nl_cols;
 };
 
+struct LeanPass;   // rk_lean.h
+
 struct PassRec {
     int kind = PK_LINE;
     int dbl = 0;
@@ -84,6 +87,7 @@ struct PassRec {
     bool use_plane_tma = false;
     int64_t plane_tma_blocks = 0;
     bool use_tma = false;
+    std::shared_ptr<const LeanPass> lean;   // taken by a lean line kernel (rk_lean.cuh)
     bool use_tc = false;           // tensor-core split-precision kernel (RK_FLAG_SPLIT_TC)
     bool pair_first = false;       // this pass and the next run as one pair launch
     PairInfo pair{};
@@ -117,6 +121,9 @@ struct DeviceTables {
     int64_t off_f[16] = {0};   // element offset of the table of L = 2^i
     int64_t off_f_r16 = 0;     // the 16-element plan of L = 8192 (RadixP<float, 8192, 1>)
     int64_t off_d[16] = {0};
+    void* lean_f = nullptr;    // stage tables of the lean passes' plans
+    void* lean_d = nullptr;
+    int64_t lean_off[2][2][2][16];   // element offset by plan set, precision, mode, log2 length
     int64_t bytes = 0;
     void* tw4hi_f = nullptr;   // float2[4096]
     void* tw4lo_f = nullptr;

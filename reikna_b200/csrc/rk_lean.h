@@ -1,0 +1,83 @@
+// Launch parameters and lookup of the lean line passes (rk_lean.cuh).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+namespace rk {
+
+// n / d for n < 2^31 as (n * m) >> sh
+struct FastDiv {
+    uint32_t d, m;
+    int32_t sh;
+};
+inline FastDiv fast_div(uint32_t d) {
+    int s = 0;
+    while ((1ull << s) < d) ++s;
+    // m = ceil(2^(31 + s) / d): the error m d - 2^(31 + s) < d <= 2^s, times n < 2^31
+    // stays below 2^(31 + s)
+    const uint64_t m = ((1ull << (31 + s)) + d - 1) / d;
+    return FastDiv{d, (uint32_t)m, 31 + s};
+}
+
+constexpr int LEAN_DIMS = 4;
+struct LeanDim {
+    FastDiv size;
+    uint32_t stride;   // bytes
+    uint32_t shift;    // index remap (r + shift) mod size
+};
+// One side: a line index splits over the dims, innermost first; position j of the line is
+// step bytes further for each j, after the remap (j + shift) mod L.
+struct LeanSide {
+    char* base;
+    LeanDim dim[LEAN_DIMS];
+    int32_t nd;
+    uint32_t step;
+    int32_t shift;
+    int32_t flags;     // SF_SCALE, SF_PRE_CONJ
+    double scale_re, scale_im;
+};
+struct LeanParams {
+    LeanSide ld, st;
+    const void* tw;
+    const void* tw4_hi;
+    const void* tw4_lo;
+    FastDiv cI, cC;    // four-step co-index of a line: (line / I) mod C
+    uint32_t nlines;
+    uint32_t tw4_mask;
+    int32_t tw4_sh;
+    // Bluestein passes (rk_lean_blue.cuh): N, the element step of the axis index
+    // a = c + j jB (columns of the three-pass form), chirp and kernel spectrum
+    uint32_t blue_n, jB;
+    const void* chirp;
+    const void* blue_k;
+};
+
+struct StageSeg {      // one stage's twiddles of a table: W_Lp^(j1 m), 1 <= m < R, j1 < J
+    int64_t off;
+    int Lp, R, J;
+};
+
+struct LeanInfo {
+    cudaError_t (*launch)(const LeanParams&, cudaStream_t);
+    cudaError_t (*prepare)();
+    void (*segments)(std::vector<StageSeg>&);
+    int tw_elems;
+    int nl;
+};
+// What a plan keeps for a pass that a lean kernel takes
+struct LeanPass {
+    LeanInfo info;
+    LeanParams prm;
+};
+
+// var 0 or 2 (transposed store); tw4: with four-step twiddles
+bool lean_info_f32(int L, int mode, int var, bool tw4, LeanInfo* out);
+bool lean_info_f64(int L, int mode, int var, bool tw4, LeanInfo* out);
+// Bluestein bodies: var 1 whole lines, 3 rows and 4 / 5 first / last columns (strided
+// lines) of the three-pass form
+bool lean_blue_info_f32(int L, int mode, int var, LeanInfo* out);
+bool lean_blue_info_f64(int L, int mode, int var, LeanInfo* out);
+
+}  // namespace rk

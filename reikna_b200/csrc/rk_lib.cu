@@ -29,10 +29,15 @@
 #include "rk_async.cuh"
 #include "rk_internal.h"
 #include "rk_kernels.cuh"
+#include "rk_lean.h"
 
 namespace rk {
 
 constexpr int ilog2_c(int n) { return n <= 1 ? 0 : 1 + ilog2_c(n / 2); }
+
+static bool lean_info(int dbl, int L, int mode, int var, bool tw4, LeanInfo* out) {
+    return dbl ? lean_info_f64(L, mode, var, tw4, out) : lean_info_f32(L, mode, var, tw4, out);
+}
 
 bool line_info_f32(int L, int mode, int var, LineInfo* out);
 bool line_info_f64(int L, int mode, int var, LineInfo* out);
@@ -68,11 +73,6 @@ __global__ void k_gen_stage(float2* f, double2* d, int Lp, int R, int J) {
     if (d) d[e] = make_double2(c, -s);
     if (f) f[e] = make_float2((float)c, (float)-s);
 }
-
-struct StageSeg {
-    int64_t off;
-    int Lp, R, J;
-};
 
 template <typename T, int L, int PL = 0> static void stage_segs(std::vector<StageSeg>& segs, int64_t base) {
     using RC = RadixP<T, L, PL>;
@@ -137,7 +137,36 @@ int device_tables(int device, DeviceTables** out) {
         memcpy(init + 2, &lim, sizeof(lim));
         CK(cudaMemcpy(t->status, init, sizeof(init), cudaMemcpyHostToDevice));
     }
-    t->bytes = nf * 8 + ndd * 16 + TW4_HALF * 48;
+    // tables of the lean passes' radix plans: a (plan set, precision, mode, length) each,
+    // set 1 the Bluestein bodies'
+    std::vector<StageSeg> lsf, lsd;
+    int64_t lnf = 0, lnd = 0;
+    for (int k = 0; k < 64; ++k) {
+        const int set = k / 64, dbl = k / 32 % 2, mode = k / 16 % 2, lg = k % 16;
+        LeanInfo li;
+        t->lean_off[set][dbl][mode][lg] = -1;
+        if (!lean_info(dbl, 1 << lg, mode, 0, false, &li)) continue;
+        int64_t& total = dbl ? lnd : lnf;
+        std::vector<StageSeg> segs;
+        li.segments(segs);
+        t->lean_off[set][dbl][mode][lg] = total;
+        for (StageSeg g : segs) {
+            g.off += total;
+            (dbl ? lsd : lsf).push_back(g);
+        }
+        total += li.tw_elems;
+    }
+    CK(cudaMalloc(&t->lean_f, std::max<int64_t>(lnf, 1) * sizeof(float2)));
+    CK(cudaMalloc(&t->lean_d, std::max<int64_t>(lnd, 1) * sizeof(double2)));
+    t->bytes = (nf + lnf) * 8 + (ndd + lnd) * 16 + TW4_HALF * 48;
+    for (const StageSeg& s : lsf) {
+        const int n = (s.R - 1) * s.J;
+        k_gen_stage<<<(n + 255) / 256, 256>>>((float2*)t->lean_f + s.off, nullptr, s.Lp, s.R, s.J);
+    }
+    for (const StageSeg& s : lsd) {
+        const int n = (s.R - 1) * s.J;
+        k_gen_stage<<<(n + 255) / 256, 256>>>(nullptr, (double2*)t->lean_d + s.off, s.Lp, s.R, s.J);
+    }
     for (const StageSeg& s : sf) {
         const int n = (s.R - 1) * s.J;
         k_gen_stage<<<(n + 255) / 256, 256>>>((float2*)t->stw_f + s.off, nullptr, s.Lp, s.R, s.J);
@@ -467,8 +496,18 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
                 // four-step n = N1 * N2: pass A over n1 (stride N2*I), pass B over n2
                 int64_t N1, N2;
                 if (I == 1) {
-                    N2 = std::min<int64_t>(256, n / 2);
-                    N1 = n / N2;
+                    if (d.flags & RK_FLAG_BATCHABLE) {
+                        // (the persistent batch kernel has bodies for these lengths)
+                        N2 = std::min<int64_t>(256, n / 2);
+                        N1 = n / N2;
+                    } else {
+                        // equal halves: the strided first pass is fastest on short lines
+                        // (complex64, 16 Mi elements: 48.5 us at 256, 51.4 at 512, 59.4
+                        // at 1024 points), the transposed second one on short lines too
+                        // (wide segments of adjacent lines; 49.2 at 512, 53.4 at 1024)
+                        N1 = int64_t(1) << (ilog2(n) / 2);
+                        N2 = n / N1;
+                    }
                     if (N1 > LM) { N1 = LM; N2 = n / N1; }
                     if (N2 > PM) {
                         set_error("1-D length beyond two-pass range");
@@ -790,6 +829,101 @@ static void setup_tma(PassRec& r, int dbl, int nsm) {
     r.nblocks = std::min<int64_t>(p.ntiles, (int64_t)nsm * per);
     r.ti = ti;
     r.use_tma = true;
+}
+
+// One side of a lean pass (rk_lean.cuh), or false where the side needs the general
+// element path: another format, padding or cropping, an additive term, a step of the
+// element index that is not the memory order, byte offsets beyond 32 bits.
+static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool unit, LeanSide* out) {
+    const int64_t esz = dbl ? 16 : 8;
+    const int32_t allowed = SF_FAST | SF_FAST2 | SF_TW4 | SF_PRE_CONJ | SF_POST_CONJ;
+    if (s.fmt != (dbl ? RK_FMT_C128 : RK_FMT_C64) || (s.flags & ~allowed)) return false;
+    if (s.ax_bound != s.ax_len || s.ax_stride < 0) return false;
+    if (p.C == 1 ? (s.cA != 0 || s.jB != 1 || s.ax_len != L) : (s.ax_shift != 0 || s.cA < 0 || s.jB < 1)) return false;
+    const int64_t step = s.jB * s.ax_stride * esz;
+    if (unit && step != esz) return false;
+    int n = 0;
+    int64_t size[2 * MAXD + 1], stride[2 * MAXD + 1], shift[2 * MAXD + 1], extent = step * (L - 1);
+    auto push = [&](int64_t sz, int64_t st, int64_t sf) {
+        if (sz == 1) return;
+        extent += (sz - 1) * st;
+        if (n && sf == 0 && shift[n - 1] == 0 && st == stride[n - 1] * size[n - 1]) {
+            size[n - 1] *= sz;
+            return;
+        }
+        size[n] = sz; stride[n] = st; shift[n] = sf;
+        ++n;
+    };
+    for (int i = s.nd_i - 1; i >= 0; --i) {
+        if (s.i_bound[i] != s.i_shape[i] || s.i_stride[i] < 0) return false;
+        push(s.i_shape[i], s.i_stride[i] * esz, s.i_shift[i]);
+    }
+    push(p.C, s.cA * s.ax_stride * esz, 0);
+    for (int i = s.nd_o - 1; i >= 0; --i) {
+        if (s.o_bound[i] != s.o_shape[i] || s.o_stride[i] < 0) return false;
+        push(s.o_shape[i], s.o_stride[i] * esz, s.o_shift[i]);
+    }
+    if (n > LEAN_DIMS || extent >= (int64_t(1) << 32)) return false;
+    LeanSide r{};
+    r.nd = n;
+    for (int i = 0; i < n; ++i) {
+        r.dim[i].size = fast_div((uint32_t)size[i]);
+        r.dim[i].stride = (uint32_t)stride[i];
+        r.dim[i].shift = (uint32_t)shift[i];
+    }
+    r.step = (uint32_t)step;
+    r.shift = s.ax_shift;
+    *out = r;
+    return true;
+}
+
+// Take the lean kernel for a plain (var 0) or transposed-store (var 2) line pass whose
+// two sides allow it.
+static int setup_lean(PassRec& r, int dbl, const DeviceTables* tabs) {
+    const PassParams& p = r.prm;
+    if (r.kind != PK_LINE || (r.var != 0 && r.var != 2) || r.user_bits) return RK_OK;
+    if (p.nlines >= (int64_t(1) << 31) || (p.ld.flags & SF_TW4)) return RK_OK;
+    const bool tw4 = p.st.flags & SF_TW4;
+    LeanInfo li;
+    LeanParams q{};
+    if (!lean_info(dbl, r.L, r.mode, r.var, tw4, &li)) return RK_OK;
+    if (!lean_side(p.ld, p, dbl, r.L, r.mode == MODE_POS, &q.ld)) return RK_OK;
+    if (!lean_side(p.st, p, dbl, r.L, r.mode == MODE_POS && r.var == 0, &q.st)) return RK_OK;
+    const int64_t off = tabs->lean_off[0][dbl][r.mode][ilog2(r.L)];
+    q.tw = dbl ? (const void*)((const double2*)tabs->lean_d + off) : (const void*)((const float2*)tabs->lean_f + off);
+    q.tw4_hi = p.tw4_hi;
+    q.tw4_lo = p.tw4_lo;
+    q.nlines = (uint32_t)p.nlines;
+    q.cI = fast_div((uint32_t)p.I);
+    q.cC = fast_div((uint32_t)p.C);
+    if (tw4) {
+        q.tw4_mask = (uint32_t)(p.tw4_N - 1);
+        q.tw4_sh = TW4_LOG - ilog2(p.tw4_N);
+        if (q.tw4_sh < 0) return RK_OK;
+    }
+    const cudaError_t e = li.prepare();
+    if (e != cudaSuccess) {
+        set_error(std::string("lean pass attributes: ") + cudaGetErrorString(e));
+        return RK_ERR_CUDA;
+    }
+    r.lean = std::make_shared<LeanPass>(LeanPass{li, q});
+    return RK_OK;
+}
+
+// The call's pointers, scales and conjugations of a lean pass.
+static void lean_call(const PassParams& p, int dbl, LeanParams& q) {
+    const int64_t esz = dbl ? 16 : 8;
+    for (int k = 0; k < 2; ++k) {
+        const Side& s = k ? p.st : p.ld;
+        LeanSide& t = k ? q.st : q.ld;
+        t.base = (char*)s.ptr + s.offset * esz;
+        t.scale_re = s.scale_re;
+        t.scale_im = s.scale_im;
+        t.flags = s.flags & SF_SCALE;
+        // without tables in between the two conjugations of a side cancel or add up; the
+        // load conjugates after its scale, the store before (as the general path does)
+        if (((s.flags & SF_PRE_CONJ) != 0) != ((s.flags & SF_POST_CONJ) != 0)) t.flags |= SF_PRE_CONJ;
+    }
 }
 
 // Sides that cannot take SF_FAST but are still the pass dtype without an index remap
@@ -1336,7 +1470,11 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             }
             r.nblocks = (pp.nlines + li.nl - 1) / li.nl;
             r.li = li;
-            if (!(desc->flags & RK_FLAG_NO_TMA) && ps.var == 0) setup_tma(r, dbl, nsm);
+            // (RK_FLAG_NO_TMA asks for the general line kernel, RK_FLAG_PAIR's launch holds
+            // its tile bodies, and the passes of a plan that may become batch members run
+            // the batch's bodies alone as well: each of them the same bits either way)
+            if (!(desc->flags & (RK_FLAG_BATCHABLE | RK_FLAG_NO_TMA | RK_FLAG_PAIR)) && (rc = setup_lean(r, dbl, tabs))) return fail(rc);
+            if (!r.lean && !(desc->flags & RK_FLAG_NO_TMA) && ps.var == 0) setup_tma(r, dbl, nsm);
             if ((desc->flags & RK_FLAG_SPLIT_TC) && tc_eligible(r)) {
                 const cudaError_t te = tc_prepare();
                 if (te != cudaSuccess) {
@@ -1345,6 +1483,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
                 }
                 r.use_tc = true;
                 r.use_tma = false;
+                r.lean.reset();
             }
         }
         plan->passes.push_back(r);
@@ -1745,6 +1884,10 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             void* args[1] = {const_cast<PassParams*>(&p)};
             const unsigned grid = (unsigned)((p.nlines + r.li.nl - 1) / r.li.nl);
             e = grid ? cudaLaunchKernel(r.user_kern, dim3(grid), dim3(r.li.nt), args, r.li.smem, st) : cudaSuccess;
+        } else if (r.lean) {
+            LeanParams q = r.lean->prm;
+            lean_call(p, r.dbl, q);
+            e = r.lean->info.launch(q, st);
         } else if (r.kind == PK_PLANE)
             e = tma[i] ? r.pti.fn(p, r.plane_tma_blocks, st) : r.pi.fn(p, r.nblocks, st);
         else if (r.use_tc)

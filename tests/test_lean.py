@@ -1,0 +1,129 @@
+"""The lean line passes (csrc/rk_lean.cuh) at the edges of their tiles, and against the
+general line kernel, which RK_FLAG_NO_TMA plans keep using."""
+
+from __future__ import annotations
+
+import math
+
+import numpy
+import pytest
+
+from helpers import fft_bound, normal_array, rel_l2
+
+gpu = pytest.mark.gpu
+
+
+def _run(x, out, axes, inverse=0, flags=0, connect=None):
+    import torch
+
+    from reikna_b200.fft import FFT
+
+    comp = FFT(x, axes=axes)
+    if connect:
+        connect(comp, out)
+    comp.compile(flags=flags)(None, out, x, inverse)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+def _check(got, x, axes, inverse=0):
+    a = x.astype(numpy.complex128)
+    ref = (numpy.fft.ifftn if inverse else numpy.fft.fftn)(a, axes=axes)
+    assert rel_l2(got, ref) < fft_bound(x.dtype, math.prod(x.shape[k] for k in axes))
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("n", [2**k for k in range(4, 15)])
+@pytest.mark.parametrize("rows", [1, 3, 33])
+def test_contiguous_lines(rng, cuda, dtype, n, rows):
+    import torch
+
+    if rows * n > 2**18:
+        rows = max(1, 2**18 // n) + 1
+    x = normal_array(rng, (rows, n), dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), (1,), inverse), x, (1,), inverse)
+    _check(_run(t, t, (1,)), x, (1,))  # in place
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("n", [2**k for k in range(1, 11)])
+@pytest.mark.parametrize("inner", [1, 5, 16, 49])
+def test_strided_lines(rng, cuda, dtype, n, inner):
+    import torch
+
+    x = normal_array(rng, (3, n, inner, 2), dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), (1,), inverse), x, (1,), inverse)
+    _check(_run(t, t, (1,)), x, (1,))
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("n", [2**k for k in range(14, 21)])
+@pytest.mark.parametrize("shape", ["rows", "strided"])
+def test_two_pass_lines(rng, cuda, dtype, n, shape):
+    import torch
+
+    if shape == "strided" and n > 2**17:
+        pytest.skip("covered by the row form's lengths")
+    rows = 3 if n < 2**19 else 1
+    s, axes = ((rows, n), (1,)) if shape == "rows" else ((n, 3), (0,))
+    x = normal_array(rng, s, dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), axes, inverse), x, axes, inverse)
+    _check(_run(t, t, axes), x, axes)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("shape,axes", [((6, 64, 32), (0,)), ((5, 64, 33), (1,)), ((4, 5, 256), (2,)), ((16, 8, 7), (0, 1)),
+                                        ((32, 32, 32), (0, 1, 2)), ((2, 3, 4, 5, 16), (1, 4))])
+def test_output_shift_and_scale(rng, cuda, dtype, shape, axes):
+    """fftshift on power-of-two axes (half the axis: a register swap), on other dims of the
+    array and on odd ones, with a complex scale."""
+    import torch
+
+    from reikna_b200 import transformations as tr
+
+    x = normal_array(rng, shape, dtype)
+    t = torch.from_numpy(x).to(cuda)
+    every = tuple(range(len(shape)))
+    factor = 0.25 - 0.5j
+
+    def connect(comp, out):
+        sh, sc = tr.fftshift(out, axes=every), tr.mul_const(out, out.cpu().numpy().dtype.type(factor))
+        comp.parameter.output.connect(sh, sh.input, shifted=sh.output)
+        comp.parameter.shifted.connect(sc, sc.input, result=sc.output)
+
+    got = _run(t, torch.empty_like(t), axes, connect=connect)
+    ref = numpy.fft.fftshift(numpy.fft.fftn(x.astype(numpy.complex128), axes=axes), axes=every) * factor
+    assert rel_l2(got, ref) < fft_bound(dtype, math.prod(shape[k] for k in axes))
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("perm", [(0, 1, 2), (2, 1, 0), (1, 0, 2), (0, 2, 1)])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_any_order_as_the_general_path(rng, cuda, dtype, perm, axis):
+    """Input and output views with permuted dims and gaps between rows: the lean route and
+    the general one agree with each other and with numpy."""
+    import torch
+
+    from reikna_b200 import _native as N
+
+    shape = (32, 64, 16)
+    base = normal_array(rng, tuple(2 * shape[p] if k == 0 else shape[p] for k, p in enumerate(perm)), dtype)
+    inv = tuple(numpy.argsort(perm))
+    t = torch.from_numpy(base).to(cuda)[::2].permute(inv)
+    x = base[::2].transpose(inv)
+    out = torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device=cuda)
+    _check(_run(t, out, (axis,)), x, (axis,))
+    lean = out.cpu().numpy()
+    general = _run(t, torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device=cuda), (axis,), flags=N.FLAG_NO_TMA)
+    assert rel_l2(lean, general) < 2 * fft_bound(dtype, shape[axis])
