@@ -70,6 +70,8 @@ struct LeanInfo {
 struct LeanPass {
     LeanInfo info;
     LeanParams prm;
+    bool blue = false;        // a Bluestein body
+    bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
 
 // var 0 or 2 (transposed store); tw4: with four-step twiddles

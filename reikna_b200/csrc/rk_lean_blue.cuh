@@ -1,0 +1,246 @@
+// Lean Bluestein passes.  With chirp[a] = exp(-i pi a^2 / N) and K the padded kernel's
+// spectrum over M, y[a] = chirp[a] (IFFT_M(FFT_M(x chirp) K))[a]; the inverse FFT runs as
+// the conjugate of a forward FFT of the conjugate.
+//
+//  * k_lean_blue: a whole line of M points a CTA.  N <= M / 2 always, so the upper half of
+//    the first FFT's inputs is zero (its first butterflies are halved) and only the lower
+//    half of the second one's outputs is computed.  The radix plans read the second FFT's
+//    inputs from the positions where the first leaves its outputs (first radix = last
+//    radix), so the multiplication by K happens in registers, without an exchange.
+//  * k_lean_mid and the chirp forms of the strided pass: M = N1 N2 in three passes.
+//    Columns of x chirp (length N1, four-step twiddles on the way out); then, row by row,
+//    FFT_N2, times K, conjugate, FFT_N2, times the same twiddles; then columns again.
+//    The spectrum is only multiplied element by element, so it may stay in the order the
+//    rows leave it in (K is laid out the same way): no transposition, and the two middle
+//    passes of the four-pass form are one.
+//
+// What bounds them is instruction issue and the barriers between stages (two FFTs of M > 2N
+// points for each line of N), so they hold 128 registers a thread at 32 elements (two
+// 256-thread CTAs an SM at M = 8192; the general kernel's paths took 255 and one CTA).
+// Measured, whole calls, against the general fused and four-pass kernels: 1000 x 3001
+// 86.0 -> 45.1 us, 1000 x 1000 over both axes 46.9 -> 28.7 us, 64 x 65521 281.9 -> 89.0 us
+// (columns 31 and 23 us, rows 40 us under ncu: issue slots 50% used, 15 to 21 of 64 warps
+// active, the rows' shared-memory and table reads 72% of the L1 data path).
+#pragma once
+#include "rk_lean.cuh"
+
+namespace rk {
+
+// v (elements i with i % R0 < R0/2 of a line; a = a0 + (tb + K(i)) jB) = x[a] chirp[a]
+// for a < N, else 0.  off excludes the position.
+template <typename T, class E, bool UNIT>
+__device__ __forceinline__ void blue_load(const LeanParams& p, uint32_t off, int tb, int a0, cplx<T>* v) {
+    using V = cplx<T>;
+    const LeanSide& s = p.ld;
+    const V* ch = reinterpret_cast<const V*>(p.chirp);
+    const int n = (int)p.blue_n, jb = UNIT ? 1 : (int)p.jB;
+    const int at = a0 + tb * jb;
+    constexpr int H = E::R0 / 2;
+    if (s.shift == 0) {
+        if constexpr (UNIT) {
+            const V* lp = reinterpret_cast<const V*>(s.base + off) + tb;
+#pragma unroll
+            for (int i = 0; i < E::RT; ++i)
+                if (i % E::R0 < H) v[i] = at + E::ik(i) < n ? lp[E::ik(i)] : cmk<V>(T(0), T(0));
+        } else {
+            const uint32_t o0 = off + (uint32_t)at * s.step, st = (uint32_t)jb * s.step;
+#pragma unroll
+            for (int i = 0; i < E::RT; ++i)
+                if (i % E::R0 < H)
+                    v[i] = at + E::ik(i) * jb < n ? *reinterpret_cast<const V*>(s.base + (o0 + (uint32_t)E::ik(i) * st))
+                                                  : cmk<V>(T(0), T(0));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i)
+            if (i % E::R0 < H) {
+                const int a = at + E::ik(i) * jb;
+                int u = a + s.shift;
+                if (u >= n) u -= n;
+                v[i] = a < n ? *reinterpret_cast<const V*>(s.base + (off + (uint32_t)u * s.step)) : cmk<V>(T(0), T(0));
+            }
+    }
+    if (s.flags & SF_SCALE) lean_scale<T, E::RT>(s, v);
+    if (s.flags & SF_PRE_CONJ) lean_conj<T, E::RT>(v);
+#pragma unroll
+    for (int i = 0; i < E::RT; ++i)
+        if (i % E::R0 < H) {
+            const int a = at + E::ik(i) * jb;
+            if (a < n) v[i] = cmul(v[i], ch[a]);
+        }
+}
+
+// Outputs i with i % RL < RL/2: chirp[a] conj(v), the inverse transform's conjugation and
+// the scale, stored for a < N.
+template <typename T, class E, bool UNIT>
+__device__ __forceinline__ void blue_store(const LeanParams& p, uint32_t off, int tb, int a0, bool ok, cplx<T>* v) {
+    using V = cplx<T>;
+    const LeanSide& s = p.st;
+    const V* ch = reinterpret_cast<const V*>(p.chirp);
+    const int n = (int)p.blue_n, jb = UNIT ? 1 : (int)p.jB;
+    const int at = a0 + tb * jb;
+    constexpr int H = E::RL / 2;
+#pragma unroll
+    for (int i = 0; i < E::RT; ++i)
+        if (i % E::RL < H) {
+            const int a = at + E::ok(i) * jb;
+            if (a < n) v[i] = cmulc(ch[a], v[i]);
+        }
+    if (s.flags & SF_PRE_CONJ) {
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i)
+            if (i % E::RL < H) v[i].y = -v[i].y;
+    }
+    if (s.flags & SF_SCALE) {
+        const T re = (T)s.scale_re, im = (T)s.scale_im;
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i)
+            if (i % E::RL < H) v[i] = im == T(0) ? cscale(v[i], re) : cmul(v[i], cmk<V>(re, im));
+    }
+    if (!ok) return;
+    if (s.shift == 0) {
+        if constexpr (UNIT) {
+            V* lp = reinterpret_cast<V*>(s.base + off) + tb;
+#pragma unroll
+            for (int i = 0; i < E::RT; ++i)
+                if (i % E::RL < H && at + E::ok(i) < n) lp[E::ok(i)] = v[i];
+        } else {
+            const uint32_t o0 = off + (uint32_t)at * s.step, st = (uint32_t)jb * s.step;
+#pragma unroll
+            for (int i = 0; i < E::RT; ++i)
+                if (i % E::RL < H && at + E::ok(i) * jb < n)
+                    *reinterpret_cast<V*>(s.base + (o0 + (uint32_t)E::ok(i) * st)) = v[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i)
+            if (i % E::RL < H) {
+                const int a = at + E::ok(i) * jb;
+                int u = a + s.shift;
+                if (u >= n) u -= n;
+                if (a < n) *reinterpret_cast<V*>(s.base + (off + (uint32_t)u * s.step)) = v[i];
+            }
+    }
+}
+
+// FFT, times K, conjugate, FFT.  kp: the line's kernel spectrum.
+template <typename T, class E, bool HALF>
+__device__ __forceinline__ void blue_core(const LeanParams& p, const cplx<T>* kp, cplx<T>* v, cplx<T>* sm, int ln, int tb) {
+    using V = cplx<T>;
+    using C = typename E::C;
+    const V* tw = reinterpret_cast<const V*>(p.tw);
+    E::template run<HALF>(v, sm, ln, tb, tw);
+    kp += tb;
+#pragma unroll
+    for (int i = 0; i < E::RT; ++i) {
+        const V k = kp[E::ok(i)];
+        v[i] = cmk<V>(v[i].x * k.x - v[i].y * k.y, -v[i].x * k.y - v[i].y * k.x);
+    }
+    if constexpr (E::NS > 1) lean_sync<C::WARP>();
+    if constexpr (E::R0 != E::RL) {
+        V* ex = sm + E::sline(ln) + E::spos(tb);
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i) ex[E::spos(E::ok(i))] = v[i];
+        lean_sync<C::WARP>();
+#pragma unroll
+        for (int i = 0; i < E::RT; ++i) v[i] = ex[E::spos(E::ik(i))];
+        lean_sync<C::WARP>();
+    }
+    E::run(v, sm, ln, tb, tw);
+}
+
+template <typename T, int L, int MODE>
+__global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, MODE, 1>::MINB))
+    k_lean_blue(const __grid_constant__ LeanParams p) {
+    using V = cplx<T>;
+    using E = LeanEngine<T, L, MODE, 1>;
+    constexpr int TPL = E::TPL, NL = E::NL;
+    extern __shared__ __align__(16) unsigned char rk_smem[];
+    V* sm = reinterpret_cast<V*>(rk_smem);
+    const int tid = threadIdx.x;
+    const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
+    const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
+    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    V v[E::RT];
+    blue_load<T, E, MODE == MODE_POS>(p, lean_offset(p.ld, line), tb, 0, v);
+    blue_core<T, E, true>(p, reinterpret_cast<const V*>(p.blue_k), v, sm, ln, tb);
+    blue_store<T, E, MODE == MODE_POS>(p, lean_offset(p.st, line), tb, 0, lt < p.nlines, v);
+}
+
+// Rows of the three-pass form: line (o, c, i) of N2 = L points; K and the twiddles of row c.
+template <typename T, int L, int MODE>
+__global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, MODE, 1>::MINB))
+    k_lean_mid(const __grid_constant__ LeanParams p) {
+    using V = cplx<T>;
+    using E = LeanEngine<T, L, MODE, 1>;
+    constexpr int TPL = E::TPL, NL = E::NL;
+    extern __shared__ __align__(16) unsigned char rk_smem[];
+    V* sm = reinterpret_cast<V*>(rk_smem);
+    const int tid = threadIdx.x;
+    const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
+    const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
+    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    const uint32_t q = fd_div(p.cI, line), c = q - fd_div(p.cC, q) * p.cC.d;
+    V v[E::RT];
+    lean_load<T, L, E::RT, MODE == MODE_POS>(p.ld, lean_offset(p.ld, line), tb, [](int i) { return E::ik(i); }, v);
+    blue_core<T, E, false>(p, reinterpret_cast<const V*>(p.blue_k) + c * (uint32_t)L, v, sm, ln, tb);
+    lean_tw4_block<T, E>(p, c, tb, v);
+    lean_store<T, L, E::RT, MODE == MODE_POS, 0>(p.st, lean_offset(p.st, line), tb, lt < p.nlines,
+                                                 [](int i) { return E::ok(i); }, v);
+}
+
+// Columns of the three-pass form.  OUT false: the first pass (chirp and zero padding on
+// the load, twiddles on the store); true: the last one (chirp on the store, a < N only).
+template <typename T, int L, bool OUT>
+__global__ void __launch_bounds__((LeanCfg<T, L, MODE_LANE, 0>::NT), (LeanCfg<T, L, MODE_LANE, 0>::MINB))
+    k_lean_cols(const __grid_constant__ LeanParams p) {
+    using V = cplx<T>;
+    using E = LeanEngine<T, L, MODE_LANE, 0>;
+    constexpr int NL = E::NL;
+    extern __shared__ __align__(16) unsigned char rk_smem[];
+    V* sm = reinterpret_cast<V*>(rk_smem);
+    const int ln = threadIdx.x % NL, tb = threadIdx.x / NL;
+    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    const uint32_t q = fd_div(p.cI, line), c = q - fd_div(p.cC, q) * p.cC.d;
+    V v[E::RT];
+    if constexpr (!OUT) {
+        blue_load<T, E, false>(p, lean_offset(p.ld, line), tb, (int)c, v);
+        E::template run<true>(v, sm, ln, tb, reinterpret_cast<const V*>(p.tw));
+        lean_tw4_block<T, E>(p, c, tb, v);
+        lean_store<T, L, E::RT, false, 0>(p.st, lean_offset(p.st, line), tb, lt < p.nlines, [](int i) { return E::ok(i); }, v);
+    } else {
+        lean_load<T, L, E::RT, false>(p.ld, lean_offset(p.ld, line), tb, [](int i) { return E::ik(i); }, v);
+        E::run(v, sm, ln, tb, reinterpret_cast<const V*>(p.tw));
+        blue_store<T, E, false>(p, lean_offset(p.st, line), tb, (int)c, lt < p.nlines, v);
+    }
+}
+
+// VAR 1: whole lines; 3: rows of the three-pass form; 4 / 5: its first / last columns
+template <typename T, int L, int MODE, int VAR> struct LeanBlueLauncher {
+    using C = LeanCfg<T, L, MODE, (VAR >= 4 ? 0 : 1)>;
+    static constexpr auto kernel() {
+        if constexpr (VAR == 1) return &k_lean_blue<T, L, MODE>;
+        else if constexpr (VAR == 3) return &k_lean_mid<T, L, MODE>;
+        else return &k_lean_cols<T, L, VAR == 5>;
+    }
+    static cudaError_t launch(const LeanParams& p, cudaStream_t st) {
+        const unsigned nb = (p.nlines + C::NL - 1) / C::NL;
+        if (nb) kernel()<<<nb, C::NT, C::SMEM, st>>>(p);
+        return cudaGetLastError();
+    }
+    static cudaError_t prepare() {
+        if (C::SMEM <= 48 * 1024) return cudaSuccess;
+        return cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    }
+    static LeanInfo info() {
+        LeanInfo r{};
+        r.launch = &launch;
+        r.prepare = &prepare;
+        r.segments = &lean_segments<C, L>;
+        r.tw_elems = LeanTw<L, typename C::P>::total();
+        r.nl = C::NL;
+        return r;
+    }
+};
+
+}  // namespace rk

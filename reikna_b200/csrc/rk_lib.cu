@@ -35,6 +35,9 @@ namespace rk {
 
 constexpr int ilog2_c(int n) { return n <= 1 ? 0 : 1 + ilog2_c(n / 2); }
 
+static bool lean_blue_info(int dbl, int L, int mode, int var, LeanInfo* out) {
+    return dbl ? lean_blue_info_f64(L, mode, var, out) : lean_blue_info_f32(L, mode, var, out);
+}
 static bool lean_info(int dbl, int L, int mode, int var, bool tw4, LeanInfo* out) {
     return dbl ? lean_info_f64(L, mode, var, tw4, out) : lean_info_f32(L, mode, var, tw4, out);
 }
@@ -141,11 +144,13 @@ int device_tables(int device, DeviceTables** out) {
     // set 1 the Bluestein bodies'
     std::vector<StageSeg> lsf, lsd;
     int64_t lnf = 0, lnd = 0;
-    for (int k = 0; k < 64; ++k) {
+    for (int k = 0; k < 128; ++k) {
         const int set = k / 64, dbl = k / 32 % 2, mode = k / 16 % 2, lg = k % 16;
         LeanInfo li;
         t->lean_off[set][dbl][mode][lg] = -1;
-        if (!lean_info(dbl, 1 << lg, mode, 0, false, &li)) continue;
+        if (!(set ? lean_blue_info(dbl, 1 << lg, mode, 1, &li) || lean_blue_info(dbl, 1 << lg, mode, 3, &li)
+                  : lean_info(dbl, 1 << lg, mode, 0, false, &li)))
+            continue;
         int64_t& total = dbl ? lnd : lnf;
         std::vector<StageSeg> segs;
         li.segments(segs);
@@ -243,14 +248,17 @@ __global__ void k_gen_window(int64_t n, int32_t w, float* f, double* d) {
     if (d) d[u] = v;
 }
 
-__global__ void k_scale_convert(const double2* src, int64_t n, double s, float2* df, double2* dd) {
+// (n1 > 1: entry k1 + n1 k2 goes to k1 (n / n1) + k2, the order the rows of the three-pass
+// Bluestein form hold the spectrum in)
+__global__ void k_scale_convert(const double2* src, int64_t n, int64_t n1, double s, float2* df, double2* dd) {
     const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     double2 v = src[k];
     v.x *= s;
     v.y *= s;
-    if (dd) dd[k] = v;
-    if (df) df[k] = make_float2((float)v.x, (float)v.y);
+    const int64_t to = k % n1 * (n / n1) + k / n1;
+    if (dd) dd[to] = v;
+    if (df) df[to] = make_float2((float)v.x, (float)v.y);
 }
 
 // ------------------------------------------------------------------------------
@@ -305,6 +313,7 @@ struct PassSpec {
     bool inplace_safe = true;
     int64_t tw4_N = 0;
     int blue_axis = -1;     // fused Bluestein kernel spectrum owner
+    int lean_var = 0;       // Bluestein body of the three-pass form (lean_blue_info), 0: none
     bool pair = false;      // with the next pass: one plane-ordered pair launch
     SideSpec ld, st;
     std::string note;
@@ -313,12 +322,13 @@ struct PassSpec {
 struct BlueAxis {
     int axis;
     int64_t N, M;
+    int64_t N1 = 1;   // > 1: the kernel spectrum in the order of the three-pass form's rows
 };
 
 struct Planned {
     std::vector<PassSpec> passes;
     std::vector<BlueAxis> blue;
-    bool need_T0 = false, need_T1 = false, need_M = false;
+    bool need_T0 = false, need_T1 = false, need_M = false, need_M1 = false;
     int64_t m_elems = 0;   // elements of an M-shaped temp
 };
 
@@ -355,6 +365,10 @@ static int half_eligible(const rk_fft_desc& d, int dbl) {
     if (ax > 0 && out.strides[ax - 1] == 1 && d.shape[ax - 1] > 1 && L <= lane_max(dbl)) return 5;
     return 0;
 }
+
+static bool lean_allowed(const rk_fft_desc& d);
+static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out);
+static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const PassSpec& last);
 
 static int plan_passes(const rk_fft_desc& d, Planned& P) {
     const int dbl = d.dtype == RK_FMT_C128;
@@ -550,7 +564,15 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
             P.blue.push_back(BlueAxis{ax, n, M});
             // a strided (lane-mode) fused Bluestein line holds up to 2048 complex64
             // points (four adjacent lines a CTA): one pass instead of four
-            const int64_t blue_lane_max = (dbl || (d.flags & RK_FLAG_BATCHABLE)) ? LM : 2048;
+            int64_t blue_lane_max = (dbl || (d.flags & RK_FLAG_BATCHABLE)) ? LM : 2048;
+            if (dbl && M == 1024 && I > 1) {
+                // (a lean body only: 1024 complex128 points, four lines a CTA)
+                PassSpec p;
+                p.axis = ax; p.L = (int)M; p.O = O; p.I = I;
+                p.ld.buf = cur; p.ld.ax_len = n; p.ld.flags = SF_CHIRP;
+                p.st.buf = last_axis ? SB_OUT : array_out(true); p.st.ax_len = n; p.st.flags = SF_PRE_CONJ | SF_CHIRP;
+                if (lean_blue_edges(d, p, p)) blue_lane_max = M;
+            }
             if ((I == 1 && M <= PM) || (I > 1 && M <= blue_lane_max)) {
                 PassSpec p;
                 p.L = (int)M; p.var = 1; p.blue_axis = ax;
@@ -598,6 +620,11 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
                 }
                 P.need_M = true;
                 P.m_elems = std::max<int64_t>(P.m_elems, O * M * I);
+                if (plan_blue3(d, P, ax, n, M, O, I, cur, last_axis ? SB_OUT : array_out(true))) {
+                    cur = P.passes.back().st.buf;
+                    continue;
+                }
+                P.need_M1 = true;
                 // forward FFT_M of chirp * x
                 PassSpec p1;
                 p1.L = (int)N1; p1.mode = MODE_LANE; p1.axis = ax; p1.O = O; p1.C = N2; p1.I = I;
@@ -834,16 +861,22 @@ static void setup_tma(PassRec& r, int dbl, int nsm) {
 // One side of a lean pass (rk_lean.cuh), or false where the side needs the general
 // element path: another format, padding or cropping, an additive term, a step of the
 // element index that is not the memory order, byte offsets beyond 32 bits.
-static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool unit, LeanSide* out) {
+//
+// blue_n: a Bluestein pass' side over the N elements of the axis itself, addressed by the
+// axis index a = c cA + j jB (the step is one element's, and the co-index c has no offset).
+static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool unit, int64_t blue_n, LeanSide* out) {
     const int64_t esz = dbl ? 16 : 8;
-    const int32_t allowed = SF_FAST | SF_FAST2 | SF_TW4 | SF_PRE_CONJ | SF_POST_CONJ;
+    const int32_t allowed = SF_FAST | SF_FAST2 | SF_TW4 | SF_PRE_CONJ | SF_POST_CONJ | (blue_n ? SF_CHIRP : 0);
     if (s.fmt != (dbl ? RK_FMT_C128 : RK_FMT_C64) || (s.flags & ~allowed)) return false;
     if (s.ax_bound != s.ax_len || s.ax_stride < 0) return false;
-    if (p.C == 1 ? (s.cA != 0 || s.jB != 1 || s.ax_len != L) : (s.ax_shift != 0 || s.cA < 0 || s.jB < 1)) return false;
-    const int64_t step = s.jB * s.ax_stride * esz;
+    if (blue_n ? s.ax_len != blue_n
+               : p.C == 1 ? (s.cA != 0 || s.jB != 1 || s.ax_len != L) : (s.ax_shift != 0 || s.cA < 0 || s.jB < 1))
+        return false;
+    const int64_t step = (blue_n ? 1 : s.jB) * s.ax_stride * esz;
     if (unit && step != esz) return false;
     int n = 0;
-    int64_t size[2 * MAXD + 1], stride[2 * MAXD + 1], shift[2 * MAXD + 1], extent = step * (L - 1);
+    int64_t size[2 * MAXD + 1], stride[2 * MAXD + 1], shift[2 * MAXD + 1];
+    int64_t extent = step * ((blue_n ? blue_n : L) - 1);
     auto push = [&](int64_t sz, int64_t st, int64_t sf) {
         if (sz == 1) return;
         extent += (sz - 1) * st;
@@ -858,7 +891,7 @@ static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool u
         if (s.i_bound[i] != s.i_shape[i] || s.i_stride[i] < 0) return false;
         push(s.i_shape[i], s.i_stride[i] * esz, s.i_shift[i]);
     }
-    push(p.C, s.cA * s.ax_stride * esz, 0);
+    push(p.C, blue_n ? 0 : s.cA * s.ax_stride * esz, 0);
     for (int i = s.nd_o - 1; i >= 0; --i) {
         if (s.o_bound[i] != s.o_shape[i] || s.o_stride[i] < 0) return false;
         push(s.o_shape[i], s.o_stride[i] * esz, s.o_shift[i]);
@@ -877,19 +910,40 @@ static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool u
     return true;
 }
 
-// Take the lean kernel for a plain (var 0) or transposed-store (var 2) line pass whose
-// two sides allow it.
-static int setup_lean(PassRec& r, int dbl, const DeviceTables* tabs) {
+// Lean kernels are not taken where a flag asks for the general tile bodies: RK_FLAG_NO_TMA
+// (the general line kernel), RK_FLAG_PAIR (whose launch holds them) and RK_FLAG_BATCHABLE
+// (passes that may become members of the persistent batch kernel run its bodies alone as
+// well).  Each of them gives the same bits either way.
+static bool lean_allowed(const rk_fft_desc& d) {
+    return !(d.flags & (RK_FLAG_BATCHABLE | RK_FLAG_NO_TMA | RK_FLAG_PAIR)) && !desc_has_user(d);
+}
+
+// Take the lean kernel for a line pass whose two sides allow it: plain (var 0), transposed
+// store (var 2), whole-line Bluestein (var 1), or a body of the three-pass form.
+static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, const DeviceTables* tabs) {
     const PassParams& p = r.prm;
-    if (r.kind != PK_LINE || (r.var != 0 && r.var != 2) || r.user_bits) return RK_OK;
+    const int bvar = ps.lean_var ? ps.lean_var : r.var == 1 ? 1 : 0;
+    const bool pos = r.mode == MODE_POS, tw4 = p.st.flags & SF_TW4;
+    if (r.kind != PK_LINE || (r.var != 0 && r.var != 1 && r.var != 2)) return RK_OK;
     if (p.nlines >= (int64_t(1) << 31) || (p.ld.flags & SF_TW4)) return RK_OK;
-    const bool tw4 = p.st.flags & SF_TW4;
-    LeanInfo li;
-    LeanParams q{};
-    if (!lean_info(dbl, r.L, r.mode, r.var, tw4, &li)) return RK_OK;
-    if (!lean_side(p.ld, p, dbl, r.L, r.mode == MODE_POS, &q.ld)) return RK_OK;
-    if (!lean_side(p.st, p, dbl, r.L, r.mode == MODE_POS && r.var == 0, &q.st)) return RK_OK;
-    const int64_t off = tabs->lean_off[0][dbl][r.mode][ilog2(r.L)];
+    auto lp = std::make_shared<LeanPass>();
+    LeanParams& q = lp->prm;
+    q = LeanParams{};
+    if (bvar) {
+        if (!lean_blue_info(dbl, r.L, r.mode, bvar, &lp->info)) return RK_OK;
+        lp->blue = true;
+        lp->fuse_next = bvar == 3;
+        q.blue_n = (uint32_t)blue_n;
+        q.jB = (uint32_t)(bvar == 4 ? p.ld.jB : bvar == 5 ? p.st.jB : 1);
+        q.chirp = bvar == 5 ? p.st.chirp : p.ld.chirp;
+        q.blue_k = p.blue_k;
+    } else if (!lean_info(dbl, r.L, r.mode, r.var, tw4, &lp->info)) {
+        return RK_OK;
+    }
+    if (!lean_side(p.ld, p, dbl, r.L, pos, bvar == 1 || bvar == 4 ? blue_n : 0, &q.ld)) return RK_OK;
+    if (!lean_side(p.st, p, dbl, r.L, pos && r.var != 2, bvar == 1 || bvar == 5 ? blue_n : 0, &q.st)) return RK_OK;
+    // (the strided first and last columns run the plain bodies' radix plans)
+    const int64_t off = tabs->lean_off[bvar == 1 || bvar == 3][dbl][r.mode][ilog2(r.L)];
     q.tw = dbl ? (const void*)((const double2*)tabs->lean_d + off) : (const void*)((const float2*)tabs->lean_f + off);
     q.tw4_hi = p.tw4_hi;
     q.tw4_lo = p.tw4_lo;
@@ -901,17 +955,90 @@ static int setup_lean(PassRec& r, int dbl, const DeviceTables* tabs) {
         q.tw4_sh = TW4_LOG - ilog2(p.tw4_N);
         if (q.tw4_sh < 0) return RK_OK;
     }
-    const cudaError_t e = li.prepare();
+    const cudaError_t e = lp->info.prepare();
     if (e != cudaSuccess) {
         set_error(std::string("lean pass attributes: ") + cudaGetErrorString(e));
         return RK_ERR_CUDA;
     }
-    r.lean = std::make_shared<LeanPass>(LeanPass{li, q});
+    r.lean = lp;
     return RK_OK;
 }
 
+static void pass_params(const rk_fft_desc& d, const PassSpec& ps, int dbl, PassParams& pp) {
+    memset(&pp, 0, sizeof(pp));
+    pp.O = ps.O; pp.C = ps.C; pp.I = ps.I;
+    pp.nlines = ps.O * ps.C * ps.I;
+    build_side(d, ps.ld, ps.axis, dbl, true, pp.ld);
+    build_side(d, ps.st, ps.kind == PK_PLANE ? ps.axis2 : ps.axis, dbl, false, pp.st);
+}
+
+// Whether the load of `first` and the store of `last` (Bluestein passes over the axis'
+// own N elements) take lean bodies.
+static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const PassSpec& last) {
+    if (!lean_allowed(d)) return false;
+    const int dbl = d.dtype == RK_FMT_C128;
+    PassParams a, b;
+    LeanSide s;
+    pass_params(d, first, dbl, a);
+    pass_params(d, last, dbl, b);
+    return a.nlines < (int64_t(1) << 31) && b.nlines < (int64_t(1) << 31) &&
+           lean_side(a.ld, a, dbl, first.L, false, first.ld.ax_len, &s) &&
+           lean_side(b.st, b, dbl, last.L, false, last.st.ax_len, &s);
+}
+
+// The three-pass form of a long Bluestein axis (rk_lean_blue.cuh), where lean bodies cover
+// it.  Its rows do the work of two of the chain's four passes in one launch.
+static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out) {
+    const int dbl = d.dtype == RK_FMT_C128;
+    const int l = ilog2(M);
+    LeanInfo li;
+    int64_t N1 = int64_t(1) << (l / 2), N2 = M / N1;
+    const int mode = I == 1 ? MODE_POS : MODE_LANE;
+    if (!dbl && I == 1 && l >= 15) {
+        // contiguous complex64 rows of 1024 points: two stages in one warp, and the second
+        // FFT reads its inputs where the first left its outputs (M = 131072, 64 lines:
+        // N2 = 1024 97 us, 512 100 us, 256 104 us)
+        N2 = l <= 20 ? 1024 : 2048;
+        N1 = M / N2;
+    }
+    if (!lean_blue_info(dbl, (int)N1, MODE_LANE, 4, &li) || !lean_blue_info(dbl, (int)N2, mode, 3, &li)) return false;
+    if (O * M * I * (dbl ? 16 : 8) >= (int64_t(1) << 32) || M > (int64_t(1) << TW4_LOG)) return false;
+    PassSpec p1;
+    p1.L = (int)N1; p1.mode = MODE_LANE; p1.axis = ax; p1.O = O; p1.C = N2; p1.I = I;
+    p1.ld.buf = cur; p1.ld.ax_len = n; p1.ld.cA = 1; p1.ld.jB = N2;
+    p1.ld.flags = SF_CHIRP; p1.ld.chirp_axis = ax;
+    p1.st.buf = SB_M0; p1.st.ax_len = M; p1.st.cA = 1; p1.st.jB = N2;
+    p1.st.flags = SF_TW4; p1.tw4_N = M;
+    p1.lean_var = 4;
+    p1.note = "bluestein-A1";
+    PassSpec p2;
+    p2.L = (int)N2; p2.mode = mode; p2.axis = ax; p2.O = O; p2.C = N1; p2.I = I;
+    p2.ld.buf = SB_M0; p2.ld.ax_len = M; p2.ld.cA = N2; p2.ld.jB = 1;
+    p2.st = p2.ld;
+    p2.st.flags = SF_TW4; p2.tw4_N = M;
+    p2.blue_axis = ax;
+    p2.lean_var = 3;
+    p2.note = "bluestein-B1";
+    PassSpec p3 = p2;   // (run by p2's launch)
+    p3.note = "bluestein-A2";
+    PassSpec p4 = p1;
+    p4.ld = p1.st;
+    p4.ld.flags = 0;
+    p4.tw4_N = 0;
+    p4.st = SideSpec();
+    p4.st.buf = out; p4.st.ax_len = n; p4.st.cA = 1; p4.st.jB = N2;
+    p4.st.flags = SF_PRE_CONJ | SF_CHIRP; p4.st.chirp_axis = ax;
+    p4.lean_var = 5;
+    p4.note = "bluestein-B2";
+    if (!lean_blue_edges(d, p1, p4)) return false;
+    for (BlueAxis& b : P.blue)
+        if (b.axis == ax) b.N1 = N1;
+    for (const PassSpec* p : {&p1, &p2, &p3, &p4}) P.passes.push_back(*p);
+    return true;
+}
+
 // The call's pointers, scales and conjugations of a lean pass.
-static void lean_call(const PassParams& p, int dbl, LeanParams& q) {
+static void lean_call(const PassParams& p, int dbl, bool blue, LeanParams& q) {
     const int64_t esz = dbl ? 16 : 8;
     for (int k = 0; k < 2; ++k) {
         const Side& s = k ? p.st : p.ld;
@@ -922,7 +1049,9 @@ static void lean_call(const PassParams& p, int dbl, LeanParams& q) {
         t.flags = s.flags & SF_SCALE;
         // without tables in between the two conjugations of a side cancel or add up; the
         // load conjugates after its scale, the store before (as the general path does)
-        if (((s.flags & SF_PRE_CONJ) != 0) != ((s.flags & SF_POST_CONJ) != 0)) t.flags |= SF_PRE_CONJ;
+        // (a Bluestein store's own conjugation, before its chirp, is part of its body)
+        const bool pre = (s.flags & SF_PRE_CONJ) && !(blue && k && (s.flags & SF_CHIRP));
+        if (pre != ((s.flags & SF_POST_CONJ) != 0)) t.flags |= SF_PRE_CONJ;
     }
 }
 
@@ -1249,7 +1378,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
     if (P.need_T1 && (rc = alloc(arr_elems * esz, &bufs[SB_T1]))) return fail(rc);
     if (P.need_M) {
         if ((rc = alloc(P.m_elems * esz, &bufs[SB_M0]))) return fail(rc);
-        if ((rc = alloc(P.m_elems * esz, &bufs[SB_M1]))) return fail(rc);
+        if (P.need_M1 && (rc = alloc(P.m_elems * esz, &bufs[SB_M1]))) return fail(rc);
     }
 
     // Bluestein tables: chirp (N) and kernel spectrum K = FFT_M(b) / M (M)
@@ -1292,7 +1421,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             krc = rk_fft_execute(kp, o, 1, in, 1, 0, nullptr, 0, nullptr);
         }
         if (krc == RK_OK) {
-            k_scale_convert<<<(unsigned)nb, 256>>>((const double2*)Kd, ba.M, 1.0 / (double)ba.M,
+            k_scale_convert<<<(unsigned)nb, 256>>>((const double2*)Kd, ba.M, ba.N1, 1.0 / (double)ba.M,
                                                    dbl ? nullptr : (float2*)K, dbl ? (double2*)K : nullptr);
             cudaError_t e3 = cudaDeviceSynchronize();
             if (e3 != cudaSuccess) {
@@ -1329,11 +1458,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
         r.inplace_safe = ps.inplace_safe;
         r.note = ps.note;
         PassParams& pp = r.prm;
-        memset(&pp, 0, sizeof(pp));
-        pp.O = ps.O; pp.C = ps.C; pp.I = ps.I;
-        pp.nlines = ps.O * ps.C * ps.I;
-        build_side(*desc, ps.ld, ps.axis, dbl, true, pp.ld);
-        build_side(*desc, ps.st, ps.kind == PK_PLANE ? ps.axis2 : ps.axis, dbl, false, pp.st);
+        pass_params(*desc, ps, dbl, pp);
         // antiperiodic transforms: W_2L^m on the first load (forward, a load-side
         // table) or after the FFT of the inverse (variant 4's rtwid), which the last
         // store's conjugation turns into W_2L^-m
@@ -1463,17 +1588,23 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             }
         } else {
             LineInfo li;
+            int64_t blue_n = 0;
+            for (const BlueAxis& ba : P.blue)
+                if (ba.axis == ps.axis) blue_n = ba.N;
+            if (lean_allowed(*desc) && (rc = setup_lean(r, ps, dbl, blue_n, tabs))) return fail(rc);
             bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);
-            if (!ok) {
+            if (!ok && !r.lean) {
                 set_error("no kernel instantiation for pass " + ps.note + " L=" + std::to_string(ps.L));
                 return fail(RK_ERR_UNSUPPORTED);
             }
-            r.nblocks = (pp.nlines + li.nl - 1) / li.nl;
-            r.li = li;
-            // (RK_FLAG_NO_TMA asks for the general line kernel, RK_FLAG_PAIR's launch holds
-            // its tile bodies, and the passes of a plan that may become batch members run
-            // the batch's bodies alone as well: each of them the same bits either way)
-            if (!(desc->flags & (RK_FLAG_BATCHABLE | RK_FLAG_NO_TMA | RK_FLAG_PAIR)) && (rc = setup_lean(r, dbl, tabs))) return fail(rc);
+            if (ps.lean_var && !r.lean) {
+                set_error("no lean body for pass " + ps.note + " L=" + std::to_string(ps.L));
+                return fail(RK_ERR_UNSUPPORTED);
+            }
+            if (ok) {
+                r.nblocks = (pp.nlines + li.nl - 1) / li.nl;
+                r.li = li;
+            }
             if (!r.lean && !(desc->flags & RK_FLAG_NO_TMA) && ps.var == 0) setup_tma(r, dbl, nsm);
             if ((desc->flags & RK_FLAG_SPLIT_TC) && tc_eligible(r)) {
                 const cudaError_t te = tc_prepare();
@@ -1516,7 +1647,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
     for (const PassRec& r : plan->passes) {
         if (r.kind == PK_PLANE)
             CK(r.pi.fn(r.prm, 0, nullptr));
-        else
+        else if (r.li.fn)
             CK(r.li.fn(r.prm, 0, nullptr));
         if (r.use_tma) CK(r.ti.fn(r.prm, 0, nullptr));
         if (r.use_plane_tma) CK(r.pti.fn(r.prm, 0, nullptr));
@@ -1886,8 +2017,19 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             e = grid ? cudaLaunchKernel(r.user_kern, dim3(grid), dim3(r.li.nt), args, r.li.smem, st) : cudaSuccess;
         } else if (r.lean) {
             LeanParams q = r.lean->prm;
-            lean_call(p, r.dbl, q);
+            lean_call(p, r.dbl, r.lean->blue, q);
             e = r.lean->info.launch(q, st);
+            if (r.lean->fuse_next) {
+                // the next pass' work is done: it records an empty interval
+                if (prof && e == cudaSuccess) {
+                    CK(cudaEventRecord(plan->prof_ev[ev + 1], st));
+                    CK(cudaEventRecord(plan->prof_ev[ev + 2], st));
+                    CK(cudaEventRecord(plan->prof_ev[ev + 3], st));
+                    ++i;
+                    continue;
+                }
+                ++i;
+            }
         } else if (r.kind == PK_PLANE)
             e = tma[i] ? r.pti.fn(p, r.plane_tma_blocks, st) : r.pi.fn(p, r.nblocks, st);
         else if (r.use_tc)

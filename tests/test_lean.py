@@ -127,3 +127,59 @@ def test_any_order_as_the_general_path(rng, cuda, dtype, perm, axis):
     lean = out.cpu().numpy()
     general = _run(t, torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device=cuda), (axis,), flags=N.FLAG_NO_TMA)
     assert rel_l2(lean, general) < 2 * fft_bound(dtype, shape[axis])
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("n", [6, 9, 15, 17, 31, 33, 63, 65, 100, 129, 255, 257, 500, 513, 1000, 1025, 2047, 2049, 4095, 4097, 8191])
+@pytest.mark.parametrize("form", ["rows", "columns"])
+def test_bluestein_lines(rng, cuda, dtype, n, form):
+    """Lengths at both ends of each padded length M, whole-line and three-pass, along
+    contiguous and strided axes."""
+    import torch
+
+    shape, axes = ((3 if n > 2000 else 37, n), (1,)) if form == "rows" else ((2, n, 5), (1,))
+    x = normal_array(rng, shape, dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), axes, inverse), x, axes, inverse)
+    _check(_run(t, t, axes), x, axes)
+
+
+@gpu
+@pytest.mark.parametrize("dtype,n,rows", [(numpy.complex64, 16001, 3), (numpy.complex64, 65521, 2), (numpy.complex64, 131101, 2),
+                                          (numpy.complex64, 300007, 1), (numpy.complex64, 600011, 1),
+                                          (numpy.complex128, 16385, 2), (numpy.complex128, 70001, 1)])
+def test_long_bluestein_lines(rng, cuda, dtype, n, rows):
+    import torch
+
+    x = normal_array(rng, (rows, n), dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), (1,), inverse), x, (1,), inverse)
+    _check(_run(t, t, (1,)), x, (1,))
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("shape,axes", [((33, 20), (0, 1)), ((3, 1001), (1,)), ((1500, 6), (0,)), ((2, 9001), (1,)), ((5, 6, 7), (0, 1, 2))])
+def test_bluestein_shift_and_scale(rng, cuda, dtype, shape, axes):
+    import torch
+
+    from reikna_b200 import transformations as tr
+
+    x = normal_array(rng, shape, dtype)
+    t = torch.from_numpy(x).to(cuda)
+    every = tuple(range(len(shape)))
+    factor = 0.25 - 0.5j
+
+    def connect(comp, out):
+        sc, sh = tr.mul_const(out, out.cpu().numpy().dtype.type(factor)), tr.fftshift(out, axes=every)
+        comp.parameter.output.connect(sc, sc.input, scaled=sc.output)
+        comp.parameter.scaled.connect(sh, sh.input, result=sh.output)
+
+    for inverse in (0, 1):
+        got = _run(t, torch.empty_like(t), axes, inverse, connect=connect)
+        ref = (numpy.fft.ifftn if inverse else numpy.fft.fftn)(x.astype(numpy.complex128), axes=axes)
+        ref = numpy.fft.fftshift(ref, axes=every) * factor
+        assert rel_l2(got, ref) < fft_bound(dtype, math.prod(shape[k] for k in axes))
