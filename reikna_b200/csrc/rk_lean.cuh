@@ -137,7 +137,7 @@ template <int L, class P> struct LeanTw {
 
 // VAR 0: plain; 1: Bluestein bodies (rk_lean_blue.cuh: two FFTs of the line with the
 // kernel spectrum between); 2: contiguous lines stored lane-fastest (transposed) through
-// shared memory
+// shared memory; 5: the same for magnitudes (rk_lean_real.cuh)
 template <typename T, int L, int MODE, int VAR> struct LeanCfg {
     using P = LeanPlan<T, L, MODE, VAR == 1>;
     using V = cplx<T>;
@@ -148,14 +148,17 @@ template <typename T, int L, int MODE, int VAR> struct LeanCfg {
     static constexpr int NT_POS = RT >= 16 ? 128 : 256;
     static constexpr int NL_POS = TPL >= NT_POS ? 1 : NT_POS / TPL;
     // transposed store: segments of 64 bytes and more a position
-    static constexpr int NL_T = NL_POS < SEG / 2 ? SEG / 2 : NL_POS;
+    static constexpr int NL_T0 = NL_POS < SEG / 2 ? SEG / 2 : NL_POS;
+    // (magnitudes are half as wide: as many lines as 256 threads hold)
+    static constexpr int NL_T1 = NL_T0 * TPL < 256 && NL_T0 < SEG ? 2 * NL_T0 : NL_T0;
+    static constexpr int NL_T = VAR == 5 ? NL_T1 : NL_T0;
     // strided lines: one 128-byte segment of adjacent lines a position, or half of one
     // where a tile would pass 64 KB
     static constexpr int NL_L0 = TPL >= 128 ? 1 : 128 / TPL;
     static constexpr int NL_L1 = NL_L0 < SEG ? SEG : NL_L0;
     static constexpr int NL_L2 = NL_L1 * L * ESZ > 65536 && NL_L1 > SEG / 2 ? SEG / 2 : NL_L1;
     static constexpr int NL_LANE = NL_L2 * L * ESZ > 65536 ? NL_L2 / 2 : NL_L2;
-    static constexpr int NL = MODE == MODE_LANE ? NL_LANE : VAR == 2 ? NL_T : NL_POS;
+    static constexpr int NL = MODE == MODE_LANE ? NL_LANE : VAR == 2 || VAR == 5 ? NL_T : NL_POS;
     static constexpr int NT = NL * TPL;
     // every line inside one warp: exchanges need only a warp barrier
     static constexpr bool WARP = MODE == MODE_POS && TPL <= 32;
@@ -167,7 +170,8 @@ template <typename T, int L, int MODE, int VAR> struct LeanCfg {
     // words: 8 / NL)
     static constexpr int D = (SEG > NL) ? SEG / NL : 1;
     static constexpr int EX = MODE == MODE_POS ? NL * LS : L * NL + (LPAD ? L / P::R[0] * NL : 0);
-    static constexpr int TR = VAR == 2 ? NL * (L + D) : 0;
+    static constexpr int TLS = L + (2 * D > 1 ? 2 * D : 2);   // magnitudes, Nyquist bin included
+    static constexpr int TR = VAR == 2 ? NL * (L + D) : VAR == 5 ? (NL * TLS + 1) / 2 : 0;
     static constexpr size_t SMEM = (P::NS > 1 || VAR != 0) ? (size_t)(EX > TR ? EX : TR) * ESZ : 0;
     // threads an SM the register budget is sized for: 32 complex64 (or 16 complex128)
     // elements a thread need 128 registers, 16 need 80, 8 and fewer 48

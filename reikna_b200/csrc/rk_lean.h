@@ -52,6 +52,18 @@ struct LeanParams {
     uint32_t blue_n, jB;
     const void* chirp;
     const void* blue_k;
+    // real passes (rk_lean_real.cuh): w_k = exp(-i pi k / L), window pairs or null, bins
+    // stored along the axis (Nyquist bin apart), LeanReal bits
+    const void* rmix;
+    const void* win;
+    uint32_t bound;
+    int32_t rflags;
+};
+enum LeanReal : int32_t {
+    LR_NYQ = 1,     // bin L is stored as well
+    LR_PAIRS = 2,   // every line of the real array starts on a pair's boundary
+    LR_NORM = 4,    // |X|^2 out, of the real type
+    LR_SQRT = 8,    // its square root
 };
 
 struct StageSeg {      // one stage's twiddles of a table: W_Lp^(j1 m), 1 <= m < R, j1 < J
@@ -71,6 +83,7 @@ struct LeanPass {
     LeanInfo info;
     LeanParams prm;
     bool blue = false;        // a Bluestein body
+    int real = 0;             // a real pass: its variant (4, 5, 6)
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
 
@@ -81,5 +94,8 @@ bool lean_info_f64(int L, int mode, int var, bool tw4, LeanInfo* out);
 // lines) of the three-pass form
 bool lean_blue_info_f32(int L, int mode, int var, LeanInfo* out);
 bool lean_blue_info_f64(int L, int mode, int var, LeanInfo* out);
+// real passes: var 6 bins or magnitudes, 5 magnitudes lane-fastest, 4 inverse
+bool lean_real_info_f32(int L, int var, LeanInfo* out);
+bool lean_real_info_f64(int L, int var, LeanInfo* out);
 
 }  // namespace rk

@@ -38,6 +38,9 @@ constexpr int ilog2_c(int n) { return n <= 1 ? 0 : 1 + ilog2_c(n / 2); }
 static bool lean_blue_info(int dbl, int L, int mode, int var, LeanInfo* out) {
     return dbl ? lean_blue_info_f64(L, mode, var, out) : lean_blue_info_f32(L, mode, var, out);
 }
+static bool lean_real_info(int dbl, int L, int var, LeanInfo* out) {
+    return dbl ? lean_real_info_f64(L, var, out) : lean_real_info_f32(L, var, out);
+}
 static bool lean_info(int dbl, int L, int mode, int var, bool tw4, LeanInfo* out) {
     return dbl ? lean_info_f64(L, mode, var, tw4, out) : lean_info_f32(L, mode, var, tw4, out);
 }
@@ -858,25 +861,13 @@ static void setup_tma(PassRec& r, int dbl, int nsm) {
     r.use_tma = true;
 }
 
-// One side of a lean pass (rk_lean.cuh), or false where the side needs the general
-// element path: another format, padding or cropping, an additive term, a step of the
-// element index that is not the memory order, byte offsets beyond 32 bits.
-//
-// blue_n: a Bluestein pass' side over the N elements of the axis itself, addressed by the
-// axis index a = c cA + j jB (the step is one element's, and the co-index c has no offset).
-static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool unit, int64_t blue_n, LeanSide* out) {
-    const int64_t esz = dbl ? 16 : 8;
-    const int32_t allowed = SF_FAST | SF_FAST2 | SF_TW4 | SF_PRE_CONJ | SF_POST_CONJ | (blue_n ? SF_CHIRP : 0);
-    if (s.fmt != (dbl ? RK_FMT_C128 : RK_FMT_C64) || (s.flags & ~allowed)) return false;
-    if (s.ax_bound != s.ax_len || s.ax_stride < 0) return false;
-    if (blue_n ? s.ax_len != blue_n
-               : p.C == 1 ? (s.cA != 0 || s.jB != 1 || s.ax_len != L) : (s.ax_shift != 0 || s.cA < 0 || s.jB < 1))
-        return false;
-    const int64_t step = (blue_n ? 1 : s.jB) * s.ax_stride * esz;
-    if (unit && step != esz) return false;
+// The dims of a lean side, innermost first (strides in bytes, cstride that of the
+// four-step co-index); false where offsets do not fit 32 bits or a dim is cropped.
+static bool lean_dims(const Side& s, const PassParams& p, int64_t esz, int64_t step, int64_t extent, int64_t cstride,
+                      LeanSide* out) {
     int n = 0;
     int64_t size[2 * MAXD + 1], stride[2 * MAXD + 1], shift[2 * MAXD + 1];
-    int64_t extent = step * ((blue_n ? blue_n : L) - 1);
+    if (step < 0 || cstride < 0) return false;
     auto push = [&](int64_t sz, int64_t st, int64_t sf) {
         if (sz == 1) return;
         extent += (sz - 1) * st;
@@ -891,7 +882,7 @@ static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool u
         if (s.i_bound[i] != s.i_shape[i] || s.i_stride[i] < 0) return false;
         push(s.i_shape[i], s.i_stride[i] * esz, s.i_shift[i]);
     }
-    push(p.C, blue_n ? 0 : s.cA * s.ax_stride * esz, 0);
+    push(p.C, cstride, 0);
     for (int i = s.nd_o - 1; i >= 0; --i) {
         if (s.o_bound[i] != s.o_shape[i] || s.o_stride[i] < 0) return false;
         push(s.o_shape[i], s.o_stride[i] * esz, s.o_shift[i]);
@@ -908,6 +899,32 @@ static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool u
     r.shift = s.ax_shift;
     *out = r;
     return true;
+}
+
+// One side of a lean pass (rk_lean.cuh), or false where the side needs the general
+// element path: another format, padding or cropping, an additive term, a step of the
+// element index that is not the memory order, byte offsets beyond 32 bits.
+//
+// blue_n: a Bluestein pass' side over the N elements of the axis itself, addressed by the
+// axis index a = c cA + j jB (the step is one element's, and the co-index c has no offset).
+static bool lean_side(const Side& s, const PassParams& p, int dbl, int L, bool unit, int64_t blue_n, LeanSide* out) {
+    const int64_t esz = dbl ? 16 : 8;
+    const int32_t allowed = SF_FAST | SF_FAST2 | SF_TW4 | SF_PRE_CONJ | SF_POST_CONJ | (blue_n ? SF_CHIRP : 0);
+    if (s.fmt != (dbl ? RK_FMT_C128 : RK_FMT_C64) || (s.flags & ~allowed) || s.ax_bound != s.ax_len) return false;
+    if (blue_n ? s.ax_len != blue_n
+               : p.C == 1 ? (s.cA != 0 || s.jB != 1 || s.ax_len != L) : (s.ax_shift != 0 || s.cA < 0 || s.jB < 1))
+        return false;
+    const int64_t step = (blue_n ? 1 : s.jB) * s.ax_stride * esz;
+    if (unit && step != esz) return false;
+    return lean_dims(s, p, esz, step, step * ((blue_n ? blue_n : L) - 1), blue_n ? 0 : s.cA * s.ax_stride * esz, out);
+}
+
+// A side of a real pass: `fmt` elements of esz bytes, contiguous lines (any step for the
+// lane-fastest store), no remap of the axis, `len` elements along it.
+static bool lean_real_side(const Side& s, const PassParams& p, int fmt, int64_t esz, bool unit, int64_t len, LeanSide* out) {
+    if (s.fmt != fmt || s.ax_shift != 0 || s.cA != 0 || s.jB != 1 || (s.flags & (SF_TAB | SF_ADD | SF_CHIRP))) return false;
+    if (unit && s.ax_stride != 1) return false;
+    return lean_dims(s, p, esz, s.ax_stride * esz, s.ax_stride * esz * (len - 1), 0, out);
 }
 
 // Lean kernels are not taken where a flag asks for the general tile bodies: RK_FLAG_NO_TMA
@@ -960,6 +977,45 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
         set_error(std::string("lean pass attributes: ") + cudaGetErrorString(e));
         return RK_ERR_CUDA;
     }
+    r.lean = lp;
+    return RK_OK;
+}
+
+// Take the lean kernel for a one-pass real transform (variants 4, 5 and 6), but for the
+// antiperiodic ones.
+static int setup_lean_real(PassRec& r, int dbl, const DeviceTables* tabs) {
+    const PassParams& p = r.prm;
+    auto lp = std::make_shared<LeanPass>();
+    LeanParams& q = lp->prm;
+    q = LeanParams{};
+    if (r.var < 4 || r.var > 6 || p.rodd || p.C != 1 || p.nlines >= (int64_t(1) << 31)) return RK_OK;
+    if (!lean_real_info(dbl, r.L, r.var, &lp->info)) return RK_OK;
+    const int cfmt = dbl ? RK_FMT_C128 : RK_FMT_C64, rfmt = dbl ? RK_FMT_F64 : RK_FMT_F32;
+    const int64_t csz = dbl ? 16 : 8, rsz = csz / 2;
+    const bool norm = p.st.fmt == rfmt;
+    if (r.var == 4) {
+        if (!p.rnyq || !lean_real_side(p.ld, p, cfmt, csz, true, r.L + 1, &q.ld) || p.st.ax_bound != r.L ||
+            !lean_real_side(p.st, p, cfmt, csz, true, r.L, &q.st))
+            return RK_OK;
+    } else {
+        if (!(p.ld.flags & SF_RPAIR) || ((p.ld.flags & SF_WINDOW) && !p.ld.win) || p.ld.ax_bound != r.L) return RK_OK;
+        if (r.var == 5 && !norm) return RK_OK;
+        if (!lean_real_side(p.ld, p, rfmt, rsz, true, 2 * (int64_t)r.L, &q.ld)) return RK_OK;
+        if (!lean_real_side(p.st, p, norm ? rfmt : cfmt, norm ? rsz : csz, r.var == 6, r.L + 1, &q.st)) return RK_OK;
+        q.win = (p.ld.flags & SF_WINDOW) ? p.ld.win : nullptr;
+    }
+    q.tw = dbl ? (const void*)((const double2*)tabs->lean_d + tabs->lean_off[0][1][MODE_POS][ilog2(r.L)])
+               : (const void*)((const float2*)tabs->lean_f + tabs->lean_off[0][0][MODE_POS][ilog2(r.L)]);
+    q.nlines = (uint32_t)p.nlines;
+    q.rmix = p.rmix;
+    q.bound = (uint32_t)p.st.ax_bound;
+    q.rflags = (p.rnyq ? LR_NYQ : 0) | (norm ? LR_NORM : 0);
+    const cudaError_t e = lp->info.prepare();
+    if (e != cudaSuccess) {
+        set_error(std::string("lean pass attributes: ") + cudaGetErrorString(e));
+        return RK_ERR_CUDA;
+    }
+    lp->real = r.var;
     r.lean = lp;
     return RK_OK;
 }
@@ -1037,12 +1093,13 @@ static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int6
     return true;
 }
 
-// The call's pointers, scales and conjugations of a lean pass.
-static void lean_call(const PassParams& p, int dbl, bool blue, LeanParams& q) {
-    const int64_t esz = dbl ? 16 : 8;
+// The call's pointers, scales and conjugations of a lean pass; false where the call needs
+// the general kernel (a norm order but 1 and 2).
+static bool lean_call(const PassParams& p, int dbl, const LeanPass& lp, LeanParams& q) {
     for (int k = 0; k < 2; ++k) {
         const Side& s = k ? p.st : p.ld;
         LeanSide& t = k ? q.st : q.ld;
+        const int64_t esz = (dbl ? 16 : 8) / (fmt_is_real(s.fmt) ? 2 : 1);
         t.base = (char*)s.ptr + s.offset * esz;
         t.scale_re = s.scale_re;
         t.scale_im = s.scale_im;
@@ -1050,9 +1107,18 @@ static void lean_call(const PassParams& p, int dbl, bool blue, LeanParams& q) {
         // without tables in between the two conjugations of a side cancel or add up; the
         // load conjugates after its scale, the store before (as the general path does)
         // (a Bluestein store's own conjugation, before its chirp, is part of its body)
-        const bool pre = (s.flags & SF_PRE_CONJ) && !(blue && k && (s.flags & SF_CHIRP));
+        const bool pre = (s.flags & SF_PRE_CONJ) && !(lp.blue && k && (s.flags & SF_CHIRP));
         if (pre != ((s.flags & SF_POST_CONJ) != 0)) t.flags |= SF_PRE_CONJ;
     }
+    if (lp.real == 5 || lp.real == 6) {
+        if ((q.rflags & LR_NORM) && p.st.post_param != 1.0 && p.st.post_param != 2.0) return false;
+        if (p.st.post_param == 1.0) q.rflags |= LR_SQRT;
+        const uintptr_t pair = dbl ? 16 : 8;
+        bool pairs = (uintptr_t)q.ld.base % pair == 0;
+        for (int d = 0; d < q.ld.nd; ++d) pairs = pairs && q.ld.dim[d].stride % pair == 0;
+        if (pairs) q.rflags |= LR_PAIRS;
+    }
+    return true;
 }
 
 // Sides that cannot take SF_FAST but are still the pass dtype without an index remap
@@ -1591,7 +1657,10 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             int64_t blue_n = 0;
             for (const BlueAxis& ba : P.blue)
                 if (ba.axis == ps.axis) blue_n = ba.N;
-            if (lean_allowed(*desc) && (rc = setup_lean(r, ps, dbl, blue_n, tabs))) return fail(rc);
+            if (lean_allowed(*desc)) {
+                rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs);
+                if (rc) return fail(rc);
+            }
             bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);
             if (!ok && !r.lean) {
                 set_error("no kernel instantiation for pass " + ps.note + " L=" + std::to_string(ps.L));
@@ -2015,9 +2084,7 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             void* args[1] = {const_cast<PassParams*>(&p)};
             const unsigned grid = (unsigned)((p.nlines + r.li.nl - 1) / r.li.nl);
             e = grid ? cudaLaunchKernel(r.user_kern, dim3(grid), dim3(r.li.nt), args, r.li.smem, st) : cudaSuccess;
-        } else if (r.lean) {
-            LeanParams q = r.lean->prm;
-            lean_call(p, r.dbl, r.lean->blue, q);
+        } else if (LeanParams q; r.lean && (q = r.lean->prm, lean_call(p, r.dbl, *r.lean, q))) {
             e = r.lean->info.launch(q, st);
             if (r.lean->fuse_next) {
                 // the next pass' work is done: it records an empty interval

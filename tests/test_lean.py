@@ -183,3 +183,59 @@ def test_bluestein_shift_and_scale(rng, cuda, dtype, shape, axes):
         ref = (numpy.fft.ifftn if inverse else numpy.fft.fftn)(x.astype(numpy.complex128), axes=axes)
         ref = numpy.fft.fftshift(ref, axes=every) * factor
         assert rel_l2(got, ref) < fft_bound(dtype, math.prod(shape[k] for k in axes))
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.float32, numpy.float64])
+@pytest.mark.parametrize("n", [2**k for k in range(5, 15)])
+@pytest.mark.parametrize("rows", [1, 37])
+def test_real_lines(rng, cuda, dtype, n, rows):
+    """Half lengths inside a warp and beyond, full and partial tiles, odd starting samples."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import IRFFT, RFFT
+
+    base = torch.from_numpy(rng.standard_normal(rows * n + 1).astype(dtype)).to(cuda)
+    cdt = torch.complex64 if dtype == numpy.float32 else torch.complex128
+    bound = fft_bound(numpy.complex64 if dtype == numpy.float32 else numpy.complex128, n)
+    for start in (0, 1):
+        t = base[start:start + rows * n].view(rows, n)
+        ref = numpy.fft.rfft(t.cpu().numpy().astype(numpy.float64), axis=1)
+        for last in (False, True):
+            out = torch.full((rows, n // 2 + (0 if last else 1)), float("nan"), dtype=cdt, device=cuda)
+            call = RFFT(ArrayMetadata((rows, n), dtype), dont_store_last=last).compile()
+            if start and dtype == numpy.float64 and n > 8192:
+                # beyond the one-pass lengths the real array is read as complex pairs
+                with pytest.raises(ValueError, match="boundary"):
+                    call(None, out, t)
+                continue
+            call(None, out, t)
+            torch.cuda.synchronize()
+            assert rel_l2(out.cpu().numpy(), ref[:, :out.shape[1]]) < bound
+    spec = torch.from_numpy(ref).to(cdt).to(cuda)
+    back = torch.empty(rows, n, dtype=t.dtype, device=cuda)
+    IRFFT(spec).compile()(None, back, spec)
+    torch.cuda.synchronize()
+    assert rel_l2(back.cpu().numpy(), numpy.fft.irfft(spec.cpu().numpy().astype(numpy.complex128), n=n, axis=1)) < bound
+
+
+@gpu
+@pytest.mark.parametrize("nfft", [2**k for k in range(5, 13)])
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("hop", ["quarter", "odd"])
+def test_spectrogram_lines(rng, cuda, nfft, transposed, hop):
+    import torch
+
+    from reikna_b200.spectrogram import frames, spectrogram
+
+    hop = nfft // 4 if hop == "quarter" else nfft // 3 | 1
+    n = nfft + 52 * hop + 3
+    x = rng.standard_normal(n).astype(numpy.float32)
+    rows, bins = frames(n, nfft, hop), nfft // 2 + 1
+    out = torch.full((bins, rows) if transposed else (rows, bins), float("nan"), dtype=torch.float32, device=cuda)
+    spectrogram(n, nfft, hop, transposed=transposed).compile()(None, out, torch.from_numpy(x).to(cuda))
+    torch.cuda.synchronize()
+    win = 0.5 * (1.0 - numpy.cos(2.0 * numpy.pi * numpy.arange(nfft) / (nfft - 1)))
+    ref = numpy.abs(numpy.fft.rfft(numpy.stack([x[k * hop:k * hop + nfft] * win for k in range(rows)]).astype(numpy.float64), axis=1))
+    assert rel_l2(out.cpu().numpy(), ref.T if transposed else ref) < fft_bound(numpy.complex64, nfft)
