@@ -157,6 +157,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, M
     constexpr int TPL = E::TPL, NL = E::NL;
     extern __shared__ __align__(16) unsigned char rk_smem[];
     V* sm = reinterpret_cast<V*>(rk_smem);
+    lean_begin();
     const int tid = threadIdx.x;
     const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, M
     constexpr int TPL = E::TPL, NL = E::NL;
     extern __shared__ __align__(16) unsigned char rk_smem[];
     V* sm = reinterpret_cast<V*>(rk_smem);
+    lean_begin();
     const int tid = threadIdx.x;
     const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
@@ -199,6 +201,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE_LANE, 0>::NT), (LeanCfg<T,
     constexpr int NL = E::NL;
     extern __shared__ __align__(16) unsigned char rk_smem[];
     V* sm = reinterpret_cast<V*>(rk_smem);
+    lean_begin();
     const int ln = threadIdx.x % NL, tb = threadIdx.x / NL;
     const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
     const uint32_t q = fd_div(p.cI, line), c = q - fd_div(p.cC, q) * p.cC.d;
@@ -224,9 +227,7 @@ template <typename T, int L, int MODE, int VAR> struct LeanBlueLauncher {
         else return &k_lean_cols<T, L, VAR == 5>;
     }
     static cudaError_t launch(const LeanParams& p, cudaStream_t st) {
-        const unsigned nb = (p.nlines + C::NL - 1) / C::NL;
-        if (nb) kernel()<<<nb, C::NT, C::SMEM, st>>>(p);
-        return cudaGetLastError();
+        return lean_launch(kernel(), (p.nlines + C::NL - 1) / C::NL, C::NT, C::SMEM, p, st);
     }
     static cudaError_t prepare() {
         if (C::SMEM <= 48 * 1024) return cudaSuccess;

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE_POS, VAR>::NT), (LeanCfg<T
     constexpr int RT = E::RT, TPL = E::TPL, NL = E::NL, H = RT / 2;
     extern __shared__ __align__(16) unsigned char rk_smem[];
     V* sm = reinterpret_cast<V*>(rk_smem);
+    lean_begin();
     const int tid = threadIdx.x, ln = tid / TPL, tb = tid % TPL;
     const uint32_t line0 = blockIdx.x * NL, lt = line0 + ln, line = min(lt, p.nlines - 1);
     V v[RT];
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE_POS, 0>::NT), (LeanCfg<T, 
     constexpr int RT = E::RT, TPL = E::TPL, NL = E::NL, H = RT / 2;
     extern __shared__ __align__(16) unsigned char rk_smem[];
     V* sm = reinterpret_cast<V*>(rk_smem);
+    lean_begin();
     const int tid = threadIdx.x, ln = tid / TPL, tb = tid % TPL;
     const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
     V y[RT], yh;   // bins tb + TPL j and their mirrors L - k; thread 0: bin L/2 apart
@@ -239,9 +241,7 @@ template <typename T, int L, int VAR> struct LeanRealLauncher {
         else return &k_lean_rpost<T, L, (VAR == 5 ? 5 : 0)>;
     }
     static cudaError_t launch(const LeanParams& p, cudaStream_t st) {
-        const unsigned nb = (p.nlines + C::NL - 1) / C::NL;
-        if (nb) kernel()<<<nb, C::NT, C::SMEM, st>>>(p);
-        return cudaGetLastError();
+        return lean_launch(kernel(), (p.nlines + C::NL - 1) / C::NL, C::NT, C::SMEM, p, st);
     }
     static cudaError_t prepare() {
         if (C::SMEM <= 48 * 1024) return cudaSuccess;
