@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <vector>
 
 namespace rk {
@@ -45,6 +46,7 @@ struct LeanParams {
     const void* tw4_lo;
     FastDiv cI, cC;    // four-step co-index of a line: (line / I) mod C
     uint32_t nlines;
+    int32_t rev;       // tiles in descending order
     uint32_t tw4_mask;
     int32_t tw4_sh;
     // Bluestein passes (rk_lean_blue.cuh): N, the element step of the axis index
@@ -84,6 +86,10 @@ struct LeanPass {
     LeanParams prm;
     bool blue = false;        // a Bluestein body
     int real = 0;             // a real pass: its variant (4, 5, 6)
+    // a plane pass: this is its rows, `second` its columns, mid the buffer between (null:
+    // the output array)
+    std::shared_ptr<const LeanPass> second;
+    void* mid = nullptr;
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
 

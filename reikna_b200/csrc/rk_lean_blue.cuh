@@ -161,7 +161,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, M
     const int tid = threadIdx.x;
     const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
-    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    const uint32_t lt = lean_tile(p) * NL + ln, line = min(lt, p.nlines - 1);
     V v[E::RT];
     blue_load<T, E, MODE == MODE_POS>(p, lean_offset(p.ld, line), tb, 0, v);
     blue_core<T, E, true>(p, reinterpret_cast<const V*>(p.blue_k), v, sm, ln, tb);
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, M
     const int tid = threadIdx.x;
     const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
-    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    const uint32_t lt = lean_tile(p) * NL + ln, line = min(lt, p.nlines - 1);
     const uint32_t q = fd_div(p.cI, line), c = q - fd_div(p.cC, q) * p.cC.d;
     V v[E::RT];
     lean_load<T, L, E::RT, MODE == MODE_POS>(p.ld, lean_offset(p.ld, line), tb, [](int i) { return E::ik(i); }, v);
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE_LANE, 0>::NT), (LeanCfg<T,
     V* sm = reinterpret_cast<V*>(rk_smem);
     lean_begin();
     const int ln = threadIdx.x % NL, tb = threadIdx.x / NL;
-    const uint32_t lt = blockIdx.x * NL + ln, line = min(lt, p.nlines - 1);
+    const uint32_t lt = lean_tile(p) * NL + ln, line = min(lt, p.nlines - 1);
     const uint32_t q = fd_div(p.cI, line), c = q - fd_div(p.cC, q) * p.cC.d;
     V v[E::RT];
     if constexpr (!OUT) {

@@ -317,6 +317,7 @@ struct PassSpec {
     int64_t tw4_N = 0;
     int blue_axis = -1;     // fused Bluestein kernel spectrum owner
     int lean_var = 0;       // Bluestein body of the three-pass form (lean_blue_info), 0: none
+    int mid = -1;           // a plane pass run as lean rows and columns: the buffer between
     bool pair = false;      // with the next pass: one plane-ordered pair launch
     SideSpec ld, st;
     std::string note;
@@ -371,6 +372,7 @@ static int half_eligible(const rk_fft_desc& d, int dbl) {
 
 static bool lean_allowed(const rk_fft_desc& d);
 static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out);
+static int plane_mid(const rk_fft_desc& d, const PassSpec& p);
 static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const PassSpec& last);
 
 static int plan_passes(const rk_fft_desc& d, Planned& P) {
@@ -471,6 +473,8 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
             const int out = last ? SB_OUT : array_out(true);
             p.st.buf = out; p.st.ax_len = p.L1; p.st.cA = 0; p.st.jB = 1;
             p.note = "plane";
+            p.mid = plane_mid(d, p);
+            if (p.mid == SB_T0) P.need_T0 = true;
             P.passes.push_back(p);
             cur = out;
             axes.erase(axes.begin(), axes.begin() + 2);
@@ -937,7 +941,7 @@ static bool lean_allowed(const rk_fft_desc& d) {
 
 // Take the lean kernel for a line pass whose two sides allow it: plain (var 0), transposed
 // store (var 2), whole-line Bluestein (var 1), or a body of the three-pass form.
-static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, const DeviceTables* tabs) {
+static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, const DeviceTables* tabs, int order) {
     const PassParams& p = r.prm;
     const int bvar = ps.lean_var ? ps.lean_var : r.var == 1 ? 1 : 0;
     const bool pos = r.mode == MODE_POS, tw4 = p.st.flags & SF_TW4;
@@ -965,6 +969,7 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
     q.tw4_hi = p.tw4_hi;
     q.tw4_lo = p.tw4_lo;
     q.nlines = (uint32_t)p.nlines;
+    q.rev = order & 1;
     q.cI = fast_div((uint32_t)p.I);
     q.cC = fast_div((uint32_t)p.C);
     if (tw4) {
@@ -1040,6 +1045,60 @@ static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const P
     return a.nlines < (int64_t(1) << 31) && b.nlines < (int64_t(1) << 31) &&
            lean_side(a.ld, a, dbl, first.L, false, first.ld.ax_len, &s) &&
            lean_side(b.st, b, dbl, last.L, false, last.st.ax_len, &s);
+}
+
+// The row and column passes a plane pass splits into, with buffer `mid` between.
+static void plane_split(const rk_fft_desc& d, const PassSpec& p, int mid, PassSpec& rows, PassSpec& cols) {
+    rows = PassSpec();
+    rows.L = p.L2; rows.mode = MODE_POS; rows.axis = p.axis;
+    rows.O = p.O * p.L1;
+    rows.ld = p.ld;
+    rows.st.buf = mid; rows.st.ax_len = p.L2;
+    cols = PassSpec();
+    cols.L = p.L1; cols.mode = MODE_LANE; cols.axis = p.axis2;
+    cols.O = p.O; cols.I = p.L2;
+    cols.ld.buf = mid; cols.ld.ax_len = p.L1;
+    cols.st = p.st;
+}
+
+// Whether a plane pass runs as two lean line passes, rows then columns, and through which
+// buffer (the output itself where the columns can be transformed in place there, else a
+// temporary); -1: the clustered kernel.  Two passes over memory at 85 to 95% of the copy
+// rate beat one at 40% (its CTAs wait for their cluster's exchange): 256 x 256 x 256
+// complex64 planes 94.3 -> 85.7 us, 1024 x 128 x 128 85.3 -> 82.1, 16 x 256 x 256 12.3 -> 9.6.
+// Where the clustered kernel keeps more in flight (64 x 64 complex64: one CTA a plane;
+// 128 x 128 complex128) it stays for arrays that L2 does not hold: 4096 x 64 x 64 71.0
+// against 81.1 us, 512 x 128 x 128 80.0 against 86.2; below, the lean passes are as fast or
+// faster (1024 x 64 x 64 21.8 against 23.3).
+static int plane_mid(const rk_fft_desc& d, const PassSpec& p) {
+    const int dbl = d.dtype == RK_FMT_C128;
+    if (!lean_allowed(d) || (d.flags & RK_FLAG_PLANE_WIDE)) return -1;
+    const int64_t bytes = p.O * p.L1 * p.L2 * (dbl ? 16 : 8);
+    if (bytes > (int64_t(64) << 20) && p.L1 == (dbl ? 128 : 64)) return -1;
+    std::vector<int> mids;
+    if (p.st.buf != SB_OUT) {
+        mids = {p.st.buf};
+    } else {
+        bool plain = true;
+        for (int i = 0; i < d.ndim; ++i) plain = plain && d.output.shift[i] == 0;
+        if (plain) mids.push_back(SB_OUT);
+        mids.push_back(SB_T0);
+    }
+    for (int mid : mids) {
+        PassSpec rows, cols;
+        plane_split(d, p, mid, rows, cols);
+        PassParams a, b;
+        LeanSide s;
+        LeanInfo li;
+        pass_params(d, rows, dbl, a);
+        pass_params(d, cols, dbl, b);
+        if (a.nlines < (int64_t(1) << 31) && lean_info(dbl, rows.L, MODE_POS, 0, false, &li) &&
+            lean_info(dbl, cols.L, MODE_LANE, 0, false, &li) && lean_side(a.ld, a, dbl, rows.L, true, 0, &s) &&
+            lean_side(a.st, a, dbl, rows.L, true, 0, &s) && lean_side(b.ld, b, dbl, cols.L, false, 0, &s) &&
+            lean_side(b.st, b, dbl, cols.L, false, 0, &s))
+            return mid;
+    }
+    return -1;
 }
 
 // The three-pass form of a long Bluestein axis (rk_lean_blue.cuh), where lean bodies cover
@@ -1506,6 +1565,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
     int64_t ntot = 1;
     for (int i = 0; i < desc->naxes; ++i) ntot *= desc->shape[desc->axes[i]];
     plan->n_total = (double)ntot;
+    int order = 0;   // lean launches so far
     for (const PassSpec& ps : P.passes) {
         PassRec r;
         r.kind = ps.kind;
@@ -1628,6 +1688,26 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
         r.L1 = ps.L1;
         r.L2 = ps.L2;
         r.axis2 = ps.axis2;
+        if (ps.kind == PK_PLANE && ps.mid >= 0) {
+            PassSpec half[2];
+            plane_split(*desc, ps, ps.mid, half[0], half[1]);
+            std::shared_ptr<LeanPass> lp[2];
+            for (int k = 0; k < 2; ++k) {
+                PassRec h;
+                h.L = half[k].L;
+                h.mode = half[k].mode;
+                pass_params(*desc, half[k], dbl, h.prm);
+                if ((rc = setup_lean(h, half[k], dbl, 0, tabs, order++))) return fail(rc);
+                if (!h.lean) {
+                    set_error("no lean body for a plane's rows or columns");
+                    return fail(RK_ERR_UNSUPPORTED);
+                }
+                lp[k] = std::make_shared<LeanPass>(*h.lean);
+            }
+            lp[0]->mid = ps.mid == SB_OUT ? nullptr : bufs[ps.mid];
+            lp[0]->second = lp[1];
+            r.lean = lp[0];
+        }
         if (ps.kind == PK_PLANE) {
             PlaneInfo pi;
             if (!plane_info(dbl, ps.L1, ps.L2, (desc->flags & RK_FLAG_PLANE_WIDE) ? 1 : 0, &pi)) {
@@ -1658,8 +1738,9 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             for (const BlueAxis& ba : P.blue)
                 if (ba.axis == ps.axis) blue_n = ba.N;
             if (lean_allowed(*desc)) {
-                rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs);
+                rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs, order);
                 if (rc) return fail(rc);
+                if (r.lean && ps.note != "bluestein-B1") ++order;   // (B1 and A2 are one launch)
             }
             bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);
             if (!ok && !r.lean) {
@@ -2085,7 +2166,17 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             const unsigned grid = (unsigned)((p.nlines + r.li.nl - 1) / r.li.nl);
             e = grid ? cudaLaunchKernel(r.user_kern, dim3(grid), dim3(r.li.nt), args, r.li.smem, st) : cudaSuccess;
         } else if (LeanParams q; r.lean && (q = r.lean->prm, lean_call(p, r.dbl, *r.lean, q))) {
-            e = r.lean->info.launch(q, st);
+            if (r.lean->second) {
+                // a plane pass: rows into the buffer between, then the columns from it
+                LeanParams c = r.lean->second->prm;
+                lean_call(p, r.dbl, *r.lean->second, c);
+                q.st.base = c.ld.base = r.lean->mid ? (char*)r.lean->mid : c.st.base;
+                q.st.flags = c.ld.flags = 0;
+                e = r.lean->info.launch(q, st);
+                if (e == cudaSuccess) e = r.lean->second->info.launch(c, st);
+            } else {
+                e = r.lean->info.launch(q, st);
+            }
             if (r.lean->fuse_next) {
                 // the next pass' work is done: it records an empty interval
                 if (prof && e == cudaSuccess) {

@@ -239,3 +239,33 @@ def test_spectrogram_lines(rng, cuda, nfft, transposed, hop):
     win = 0.5 * (1.0 - numpy.cos(2.0 * numpy.pi * numpy.arange(nfft) / (nfft - 1)))
     ref = numpy.abs(numpy.fft.rfft(numpy.stack([x[k * hop:k * hop + nfft] * win for k in range(rows)]).astype(numpy.float64), axis=1))
     assert rel_l2(out.cpu().numpy(), ref.T if transposed else ref) < fft_bound(numpy.complex64, nfft)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("shape", [(3, 64, 64), (2, 128, 128), (3, 256, 256), (5, 128, 128, 2), (2, 3, 256, 256)])
+@pytest.mark.parametrize("shift", [False, True])
+def test_plane_as_rows_and_columns(rng, cuda, dtype, shape, shift):
+    """Planes whose columns are transformed in place in the output, and through a
+    temporary where the output is remapped; out of place, in place and strided."""
+    import torch
+
+    from reikna_b200 import transformations as tr
+
+    axes = (1, 2) if shape[-1] == 2 else (len(shape) - 2, len(shape) - 1)
+    x = normal_array(rng, shape, dtype)
+    t = torch.from_numpy(x).to(cuda)
+
+    def connect(comp, out):
+        sh = tr.fftshift(out, axes=axes)
+        comp.parameter.output.connect(sh, sh.input, shifted=sh.output)
+
+    for inverse in (0, 1):
+        ref = (numpy.fft.ifftn if inverse else numpy.fft.fftn)(x.astype(numpy.complex128), axes=axes)
+        if shift:
+            ref = numpy.fft.fftshift(ref, axes=axes)
+        for out in (torch.empty_like(t), t.clone()):
+            src = t if out.data_ptr() != t.data_ptr() else out
+            assert rel_l2(_run(src, out, axes, inverse, connect=connect if shift else None), ref) < fft_bound(dtype, shape[axes[0]] * shape[axes[1]])
+        same = t.clone()
+        assert rel_l2(_run(same, same, axes, inverse, connect=connect if shift else None), ref) < fft_bound(dtype, shape[axes[0]] * shape[axes[1]])
