@@ -183,6 +183,10 @@ RK_API int rk_fft_execute(rk_fft_plan* plan, void* const* outputs, int32_t n_out
                    const void* const* inputs, int32_t n_inputs, int32_t inverse,
                    const double* scalars, int32_t n_scalars, void* stream);
 
+/* rk_fft_execute of a plan with one output and one input array and no scalars, with less
+ * work on the host per call. */
+RK_API int rk_fft_call(rk_fft_plan* plan, void* output, const void* input, int32_t inverse, void* stream);
+
 RK_API int rk_fft_plan_destroy(rk_fft_plan* plan);
 
 /*

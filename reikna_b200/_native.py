@@ -56,6 +56,7 @@ EXPORTED = (
     "rk_edge_init",
     "rk_fft_plan_create",
     "rk_fft_execute",
+    "rk_fft_call",
     "rk_fft_execute_user",
     "rk_fft_plan_pass_info",
     "rk_fft_plan_set_pass_kernel",
@@ -182,6 +183,7 @@ def lib() -> ctypes.CDLL:
             ctypes.c_int32,
             vp,
         ]
+        L.rk_fft_call.argtypes = [vp, vp, vp, ctypes.c_int32, vp]
         L.rk_fft_plan_destroy.argtypes = [vp]
         u64p = ctypes.POINTER(ctypes.c_uint64)
         L.rk_fft_execute_user.argtypes = [vp, ctypes.POINTER(vp), ctypes.c_int32, ctypes.POINTER(vp), ctypes.c_int32,
@@ -334,6 +336,12 @@ class Plan:
             sc = (ctypes.c_double * len(flat))(*flat)
         rc = lib().rk_fft_execute(self._h, outs_a, len(outs), ins_a, len(ins), int(inverse), sc, len(scalars),
                                   stream)
+        if rc:
+            check(rc)
+
+    def call(self, out: int, inp: int, inverse: int, stream: int) -> None:
+        """``execute`` with one array each way and no scalars."""
+        rc = _lib.rk_fft_call(self._h, out, inp, inverse, stream)
         if rc:
             check(rc)
 

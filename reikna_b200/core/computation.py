@@ -207,6 +207,54 @@ def array_pointer(arr, annotation) -> int:
     return int(arr.data_ptr())
 
 
+def _direct_call(names, plan, out_check, in_check, out_name, in_name, inverse):
+    """The common call (positional arguments, one array each way, no scalars but the
+    direction) without the dictionary, the numpy scalar and the pointer arrays of the
+    general path: 7.7 -> 4.0 us a call of a one-kernel plan.  Returns False, before anything
+    is queued, for any other call and for arrays that do not match; the general path then
+    binds and checks it.  ``inverse``: the direction of computations without that
+    parameter, None to take it from the call."""
+    import torch
+
+    total = len(names)
+    io, ii = names.index(out_name), names.index(in_name)
+    iv = total - 1 if inverse is None else -1
+    if inverse is None and (total != 3 or names[iv] != "inverse" or iv in (io, ii)):
+        return None
+    if inverse is not None and total != 2:
+        return None
+    odt, oshape, ostrides = out_check.tdtype, out_check.shape, out_check.strides
+    idt, ishape, istrides = in_check.tdtype, in_check.shape, in_check.strides
+    device, raw = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if device is None or raw is None:
+        return None
+
+    def call(stream, args) -> bool:
+        if len(args) == total:
+            inv = inverse if iv < 0 else args[iv]
+            if inv != 0 and inv != 1 or type(inv) is not int:
+                return False
+        elif iv >= 0 and len(args) == total - 1:
+            inv = 0
+        else:
+            return False
+        out, inp = args[io], args[ii]
+        try:
+            if not (out.is_cuda and inp.is_cuda and out.dtype is odt and inp.dtype is idt and out.shape == oshape
+                    and inp.shape == ishape and out.stride() == ostrides and inp.stride() == istrides):
+                return False
+        except AttributeError:
+            return False
+        if stream is None:
+            stream = raw(device())
+        elif type(stream) is not int:
+            stream = stream_handle(stream)
+        plan.call(out.data_ptr(), inp.data_ptr(), inv, stream)
+        return True
+
+    return call
+
+
 class ComputationCallable:
     """A compiled computation: ``callable(stream, *args, **kwds)``; asynchronous."""
 
@@ -221,6 +269,8 @@ class ComputationCallable:
         self._defaults = [p.default for p in params]
         self._scalar_dt = [p.annotation.dtype if p.annotation.is_scalar() else None for p in params]
         self._required = sum(1 for p in params if p.default is inspect.Parameter.empty)
+        direct = getattr(runner, "direct", None)
+        self._direct = _direct_call(self._names, *direct) if direct is not None else None
 
     def _bind_positional(self, args) -> dict | None:
         n = len(args)
@@ -242,6 +292,8 @@ class ComputationCallable:
         return out
 
     def __call__(self, stream, *args, **kwds):
+        if self._direct is not None and not kwds and self._direct(stream, args):
+            return None
         bound = None if kwds else self._bind_positional(args)
         if bound is None:
             bound = self.signature.bind_with_defaults(args, kwds, cast=True).arguments

@@ -64,7 +64,8 @@ struct PairInfo {
     int nl_rows, nl_cols;
 };
 
-struct LeanPass;   // rk_lean.h
+struct LeanPass;    // rk_lean.h
+struct LeanChain;
 
 struct PassRec {
     int kind = PK_LINE;
@@ -155,4 +156,6 @@ struct rk_fft_plan {
     // per-pass event profiling (rk_fft_profile)
     std::vector<cudaEvent_t> prof_ev;   // 2 * passes * max_calls
     int32_t prof_max = 0, prof_used = 0;
+    // launches of both directions where every pass is lean and no scalar is set per call
+    std::shared_ptr<const rk::LeanChain> chain[2];
 };

@@ -93,6 +93,18 @@ struct LeanPass {
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
 
+// A plan's launches of one direction, but for the user's pointers
+struct LeanChain {
+    enum { FIXED = 0, INPUT = 1, OUTPUT = 2 };
+    struct Item {
+        cudaError_t (*launch)(const LeanParams&, cudaStream_t);
+        LeanParams prm;           // sides of the user's arrays hold their offset from the pointer
+        int32_t ld = FIXED, st = FIXED;
+        uint32_t pair = 0;        // drop LR_PAIRS where the load's base is off this boundary
+    };
+    std::vector<Item> items;
+};
+
 // var 0 or 2 (transposed store); tw4: with four-step twiddles
 bool lean_info_f32(int L, int mode, int var, bool tw4, LeanInfo* out);
 bool lean_info_f64(int L, int mode, int var, bool tw4, LeanInfo* out);

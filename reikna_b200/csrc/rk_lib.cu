@@ -1321,6 +1321,71 @@ static int64_t edge_extent_bytes(const rk_edge& e, int second) {
 
 }  // namespace rk
 
+namespace rk {
+int build_call_params(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs, const void* const* inputs,
+                      int32_t n_inputs, int32_t inverse, const double* scalars, int32_t n_scalars, cudaStream_t st,
+                      std::vector<PassParams>& out, std::vector<char>* tma_ok, const uint64_t* user_in,
+                      int32_t n_user_in, const uint64_t* user_out, int32_t n_user_out);
+
+// The launches of one direction of a plan whose passes are all lean and whose edges take
+// one array each and no scalars: what rk_fft_call does per call is then to fill in the
+// pointers (building each pass' general parameters, 1.7 KB a pass, and the conversion
+// from them took about a microsecond a call).
+static std::shared_ptr<const LeanChain> build_chain(rk_fft_plan* plan, int inverse) {
+    const rk_fft_desc& d = plan->desc;
+    if (fmt_arrays(d.input.format) != 1 || fmt_arrays(d.output.format) != 1) return nullptr;
+    for (const rk_edge* e : {&d.input, &d.output})
+        if (e->scale_slot >= 0 || e->scale_div_slot >= 0 || e->add_slot >= 0 || e->post_slot >= 0) return nullptr;
+    if ((d.flags & RK_FLAG_REAL_POST && inverse) || (d.flags & RK_FLAG_REAL_PRE && !inverse)) return nullptr;
+    for (const PassRec& r : plan->passes)
+        if (!r.lean || r.pair_first || r.user_kern) return nullptr;
+    // stand-ins for the user's pointers, aligned and apart
+    char *in = (char*)0x10000000, *out = (char*)0x20000000;
+    void* outs[1] = {out};
+    const void* ins[1] = {in};
+    std::vector<PassParams> prm;
+    if (build_call_params(plan, outs, 1, ins, 1, inverse, nullptr, 0, nullptr, prm, nullptr, nullptr, 0, nullptr, 0) != RK_OK)
+        return nullptr;
+    auto chain = std::make_shared<LeanChain>();
+    auto rebase = [&](LeanSide& s, int kind) {
+        if (kind != LeanChain::FIXED) s.base = (char*)nullptr + (s.base - (kind == LeanChain::INPUT ? in : out));
+    };
+    for (size_t i = 0; i < plan->passes.size(); ++i) {
+        const PassRec& r = plan->passes[i];
+        const LeanPass& lp = *r.lean;
+        LeanChain::Item a;
+        a.prm = lp.prm;
+        if (!lean_call(prm[i], r.dbl, lp, a.prm)) return nullptr;
+        a.launch = lp.info.launch;
+        a.ld = r.ld_edge ? LeanChain::INPUT : LeanChain::FIXED;
+        a.st = r.st_edge ? LeanChain::OUTPUT : LeanChain::FIXED;
+        if (a.prm.rflags & LR_PAIRS) a.pair = r.dbl ? 16 : 8;
+        if (lp.second) {
+            LeanChain::Item c = a;
+            c.prm = lp.second->prm;
+            lean_call(prm[i], r.dbl, *lp.second, c.prm);
+            c.launch = lp.second->info.launch;
+            a.st = c.ld = lp.mid ? LeanChain::FIXED : c.st;
+            a.prm.st.base = c.prm.ld.base = lp.mid ? (char*)lp.mid : c.prm.st.base;
+            a.prm.st.flags = c.prm.ld.flags = 0;
+            rebase(a.prm.ld, a.ld);
+            rebase(a.prm.st, a.st);
+            rebase(c.prm.ld, c.ld);
+            rebase(c.prm.st, c.st);
+            chain->items.push_back(a);
+            chain->items.push_back(c);
+            continue;
+        }
+        rebase(a.prm.ld, a.ld);
+        rebase(a.prm.st, a.st);
+        chain->items.push_back(a);
+        if (lp.fuse_next) ++i;
+    }
+    return chain;
+}
+
+}  // namespace rk
+
 using namespace rk;
 
 // ------------------------------------------------------------------------------
@@ -1803,6 +1868,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
         if (r.use_plane_tma) CK(r.pti.fn(r.prm, 0, nullptr));
     }
     CK(cudaDeviceSynchronize());
+    for (int inverse = 0; inverse < 2; ++inverse) plan->chain[inverse] = build_chain(plan, inverse);
     *out = plan;
     return RK_OK;
 }
@@ -2110,6 +2176,24 @@ int rk_fft_execute(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs, c
                    int32_t n_inputs, int32_t inverse, const double* scalars, int32_t n_scalars, void* stream) {
     return rk_fft_execute_user(plan, outputs, n_outputs, inputs, n_inputs, inverse, scalars, n_scalars, nullptr, 0,
                                nullptr, 0, stream);
+}
+
+int rk_fft_call(rk_fft_plan* plan, void* output, const void* input, int32_t inverse, void* stream) {
+    const LeanChain* chain = plan ? plan->chain[inverse ? 1 : 0].get() : nullptr;
+    if (!chain || !output || !input || plan->prof_used < plan->prof_max || (plan->alias_hazard && input == output))
+        return rk_fft_execute(plan, &output, 1, &input, 1, inverse, nullptr, 0, stream);
+    for (const LeanChain::Item& it : chain->items) {
+        LeanParams q = it.prm;
+        if (it.ld) q.ld.base = (it.ld == LeanChain::INPUT ? (char*)const_cast<void*>(input) : (char*)output) + (intptr_t)q.ld.base;
+        if (it.st) q.st.base = (char*)output + (intptr_t)q.st.base;
+        if (it.pair && (uintptr_t)q.ld.base % it.pair) q.rflags &= ~LR_PAIRS;
+        const cudaError_t e = it.launch(q, (cudaStream_t)stream);
+        if (e != cudaSuccess) {
+            set_error(std::string("kernel launch failed: ") + cudaGetErrorString(e));
+            return RK_ERR_CUDA;
+        }
+    }
+    return RK_OK;
 }
 
 int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs, const void* const* inputs,

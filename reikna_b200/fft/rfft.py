@@ -25,7 +25,7 @@ from __future__ import annotations
 import numpy
 
 from .. import _native as N
-from ..core.computation import Computation, array_pointer
+from ..core.computation import ArrayCheck, Computation, array_pointer
 from ..core.signature import Annotation, ArrayMetadata, Parameter, Type
 from .fft import FFT
 
@@ -139,7 +139,7 @@ def _fused_runner(fused, ann, esz: int, inverse: int, real_side: str):
         inp = array_pointer(args["input"], ann["input"])
         if (inp if real_side == "input" else out) % esz:
             raise ValueError("the real array must start on a boundary of its complex pair type")
-        fused.execute([out], [inp], inverse=inverse, stream=stream)
+        fused.call(out, inp, inverse, stream)
 
     run.launches = fused.launches
     run.plan = fused
@@ -171,17 +171,18 @@ class RFFT(Computation):
             def run(stream: int, args):
                 out = array_pointer(args["output"], ann["output"])
                 inp = array_pointer(args["input"], ann["input"])
-                route.execute([out], [inp], inverse=0, stream=stream)
+                route.call(out, inp, 0, stream)
 
             run.launches = route.launches
             run.plan = route
+            run.direct = (route, ArrayCheck(ann["output"]), ArrayCheck(ann["input"]), "output", "input", 0)
             return run
         h = _Half(device, meta.shape[:-1], half, cdt)
 
         def runner(stream: int, args):
             out = array_pointer(args["output"], ann["output"])
             inp = h.aligned(array_pointer(args["input"], ann["input"]))
-            h.plan.execute([h.temp.data_ptr()], [inp], inverse=0, stream=stream)
+            h.plan.call(h.temp.data_ptr(), inp, 0, stream)
             N.check(N.lib().rk_rfft_post(out, h.temp.data_ptr(), h.table.data_ptr(), h.fmt, h.half, h.batch,
                                          store_last, stream))
 
@@ -216,7 +217,7 @@ class IRFFT(Computation):
             out = h.aligned(array_pointer(args["output"], ann["output"]))
             inp = array_pointer(args["input"], ann["input"])
             N.check(N.lib().rk_irfft_pre(h.temp.data_ptr(), inp, h.table.data_ptr(), h.fmt, h.half, h.batch, stream))
-            h.plan.execute([out], [h.temp.data_ptr()], inverse=1, stream=stream)
+            h.plan.call(out, h.temp.data_ptr(), 1, stream)
 
         runner.launches = h.plan.launches + 1
         runner.half = h
@@ -262,7 +263,7 @@ class APRFFT(Computation):
             inp = h.aligned(array_pointer(args["input"], ann["input"]))
             t = h.temp.data_ptr()
             N.check(lib.rk_aprfft_twiddle(t, inp, h.table.data_ptr(), h.fmt, h.half, h.batch, 0, stream))
-            h.plan.execute([t], [t], inverse=0, stream=stream)
+            h.plan.call(t, t, 0, stream)
             N.check(lib.rk_aprfft_post(out, t, h.table.data_ptr(), h.fmt, h.half, h.batch, stream))
 
         runner.launches = h.plan.launches + 2
@@ -302,7 +303,7 @@ class IAPRFFT(Computation):
             inp = array_pointer(args["input"], ann["input"])
             t = h.temp.data_ptr()
             N.check(lib.rk_iaprfft_pre(t, inp, h.table.data_ptr(), h.fmt, h.half, h.batch, stream))
-            h.plan.execute([out], [t], inverse=1, stream=stream)
+            h.plan.call(out, t, 1, stream)
             N.check(lib.rk_aprfft_twiddle(out, out, h.table.data_ptr(), h.fmt, h.half, h.batch, 1, stream))
 
         runner.launches = h.plan.launches + 2
