@@ -28,6 +28,25 @@ struct LeanDim {
     uint32_t stride;   // bytes
     uint32_t shift;    // index remap (r + shift) mod size
 };
+// Stage of a mixed-radix pass (rk_lean_mix.cuh): radix R after P = the product of the
+// earlier ones, nb = L / R butterflies a line, J = nb / P twiddle groups
+struct MixStage {
+    uint32_t R, P, nb, J, tw;
+    FastDiv bdiv, pdiv;   // by nb, by P
+};
+constexpr int MIX_STAGES = 4;
+constexpr int MIX_SMEM = 200 * 1024;   // dynamic shared memory of a CTA at most
+struct MixPlan {
+    uint32_t n;
+    int32_t ns;
+    uint32_t nl, lsh;      // lines a tile (strided: a power of two, and its logarithm)
+    uint32_t buf, pitch;   // elements of a buffer and of a line in it
+    uint32_t pad;          // one pad word for each R0 positions (r0 divides by R0)
+    uint32_t inplace;      // a thread has at most one butterfly a stage
+    FastDiv r0;
+    MixStage stage[MIX_STAGES];
+};
+
 // One side: a line index splits over the dims, innermost first; position j of the line is
 // step bytes further for each j, after the remap (j + shift) mod L.
 struct LeanSide {
@@ -60,6 +79,9 @@ struct LeanParams {
     const void* win;
     uint32_t bound;
     int32_t rflags;
+    // mixed-radix passes: the plan on the device, lines and threads a CTA, shared memory
+    const MixPlan* mix;
+    uint32_t mix_nl, mix_nt, mix_smem;
 };
 enum LeanReal : int32_t {
     LR_NYQ = 1,     // bin L is stored as well
@@ -92,6 +114,10 @@ struct LeanPass {
     void* mid = nullptr;
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
+
+// Mixed-radix passes: the kernel of a mode
+void lean_mix_info_f32(int mode, LeanInfo* out);
+void lean_mix_info_f64(int mode, LeanInfo* out);
 
 // A plan's launches of one direction, but for the user's pointers
 struct LeanChain {

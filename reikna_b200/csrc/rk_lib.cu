@@ -15,6 +15,7 @@
 //     rows and columns through distributed shared memory (rk_plane.cu).
 #include <cuda_runtime.h>
 #include <math.h>
+#include <cmath>
 #include <stdio.h>
 #include <string.h>
 
@@ -317,6 +318,7 @@ struct PassSpec {
     int64_t tw4_N = 0;
     int blue_axis = -1;     // fused Bluestein kernel spectrum owner
     int lean_var = 0;       // Bluestein body of the three-pass form (lean_blue_info), 0: none
+    bool mixed = false;     // mixed-radix pass of L points (rk_lean_mix.cuh)
     int mid = -1;           // a plane pass run as lean rows and columns: the buffer between
     bool pair = false;      // with the next pass: one plane-ordered pair launch
     SideSpec ld, st;
@@ -373,6 +375,7 @@ static int half_eligible(const rk_fft_desc& d, int dbl) {
 static bool lean_allowed(const rk_fft_desc& d);
 static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out);
 static int plane_mid(const rk_fft_desc& d, const PassSpec& p);
+static bool mix_ok(const rk_fft_desc& d, const PassSpec& p);
 static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const PassSpec& last);
 
 static int plan_passes(const rk_fft_desc& d, Planned& P) {
@@ -567,6 +570,24 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
                 cur = out;
             }
         } else {
+            {
+                // small prime factors: the FFT of the length itself in one pass
+                PassSpec p;
+                p.L = (int)n;
+                p.mode = I == 1 ? MODE_POS : MODE_LANE;
+                p.axis = ax;
+                p.O = O; p.I = I;
+                p.ld.buf = cur; p.ld.ax_len = n;
+                const int out = last_axis ? SB_OUT : array_out(true);
+                p.st.buf = out; p.st.ax_len = n;
+                p.note = "mixed";
+                p.mixed = true;
+                if (!real_flags && !(d.flags & (RK_FLAG_R16 | RK_FLAG_BLUE_PAIR)) && mix_ok(d, p)) {
+                    P.passes.push_back(p);
+                    cur = out;
+                    continue;
+                }
+            }
             const int64_t M = 2 * bpow2(n);
             P.blue.push_back(BlueAxis{ax, n, M});
             // a strided (lane-mode) fused Bluestein line holds up to 2048 complex64
@@ -870,7 +891,7 @@ static void setup_tma(PassRec& r, int dbl, int nsm) {
 static bool lean_dims(const Side& s, const PassParams& p, int64_t esz, int64_t step, int64_t extent, int64_t cstride,
                       LeanSide* out) {
     int n = 0;
-    int64_t size[2 * MAXD + 1], stride[2 * MAXD + 1], shift[2 * MAXD + 1];
+    int64_t size[2 * MAXD + 1] = {}, stride[2 * MAXD + 1] = {}, shift[2 * MAXD + 1] = {};
     if (step < 0 || cstride < 0) return false;
     auto push = [&](int64_t sz, int64_t st, int64_t sf) {
         if (sz == 1) return;
@@ -1045,6 +1066,154 @@ static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const P
     return a.nlines < (int64_t(1) << 31) && b.nlines < (int64_t(1) << 31) &&
            lean_side(a.ld, a, dbl, first.L, false, first.ld.ax_len, &s) &&
            lean_side(b.st, b, dbl, last.L, false, last.st.ax_len, &s);
+}
+
+// Radices (at most 16) of a mixed-radix plan of n points, or 0: the split with the least
+// work, counting per element what a stage costs (shared memory, twiddle, addresses: 14) and
+// what its DFT does (arithmetic grows with the largest prime; there is none for 13).  An odd radix goes first
+// where there is one (its stride meets every bank), then the larger ones.
+static int mix_radices(int64_t n, int* r) {
+    static const int cost[17] = {0, 0, 2, 5, 4, 8, 7, 12, 7, 10, 10, 22, 9, 0, 14, 13, 10};
+    if (n < 6 || n > 8192) return 0;
+    int best = 1 << 30, nbest = 0, cur[MIX_STAGES];
+    auto search = [&](auto&& self, int64_t left, int at, int top, int sum) -> void {
+        if (left == 1) {
+            if (at >= 2 && sum < best) {
+                best = sum;
+                nbest = at;
+                std::copy(cur, cur + at, r);
+            }
+            return;
+        }
+        if (at == MIX_STAGES) return;
+        for (int R = top; R >= 2; --R)
+            if (left % R == 0 && R != 13) {
+                cur[at] = R;
+                self(self, left / R, at + 1, R, sum + 14 + cost[R]);
+            }
+    };
+    search(search, n, 0, 16, 0);
+    for (int i = 0; i < nbest; ++i)
+        if (r[i] % 2) {
+            std::rotate(r, r + i, r + i + 1);
+            break;
+        }
+    return nbest;
+}
+
+// Tile of a mixed-radix pass: lines and threads a CTA, from the share of threads that hold
+// a butterfly in every stage, the CTAs an SM (registers: 768 complex64 threads, 512
+// complex128; shared memory) and, for strided lines, the width of their segments.
+static bool mix_tile(int64_t n, int dbl, int mode, int64_t nlines, int nsm, MixPlan& x, uint32_t* nt_out, uint32_t* smem_out) {
+    int r[MIX_STAGES];
+    const int ns = mix_radices(n, r);
+    if (!ns) return false;
+    x = MixPlan{};
+    x.n = (uint32_t)n;
+    x.ns = ns;
+    x.pad = mode == MODE_POS && r[0] % 2 == 0;
+    x.r0 = fast_div((uint32_t)r[0]);
+    x.pitch = (uint32_t)(n + (x.pad ? n / r[0] : 0));
+    uint32_t P = 1, tw = 0;
+    for (int s = 0; s < ns; ++s) {
+        MixStage& g = x.stage[s];
+        g.R = (uint32_t)r[s];
+        g.P = P;
+        g.nb = (uint32_t)(n / r[s]);
+        g.J = g.nb / P;
+        g.tw = tw;
+        g.bdiv = fast_div(g.nb);
+        g.pdiv = fast_div(P);
+        tw += (g.R - 1) * g.J;
+        P *= g.R;
+    }
+    const int esz = dbl ? 16 : 8, max_nt = dbl ? 256 : 384, sm_threads = dbl ? 512 : 768;
+    double best = 1e30;
+    for (uint32_t nl = 1; nl <= 256; mode == MODE_LANE ? nl *= 2 : ++nl) {
+        if (mode == MODE_LANE && nl * esz > 128) break;
+        if (nl > 1 && nl * n > 4096 && mode == MODE_POS) break;
+        for (uint32_t nt = 64; nt <= (uint32_t)max_nt; nt += 32) {
+            double slots = 0;
+            bool one = true;
+            for (int s = 0; s < ns; ++s) {
+                const uint64_t total = (uint64_t)x.stage[s].nb * nl, rounds = (total + nt - 1) / nt;
+                slots += (double)rounds * nt * (14.0 * x.stage[s].R);
+                one = one && rounds == 1;
+            }
+            const uint64_t buf = mode == MODE_LANE ? (uint64_t)n * nl : (uint64_t)x.pitch * nl;
+            const uint64_t smem = buf * esz * (one || ns < 3 ? 1 : 2) + nl * 8;
+            if (smem > MIX_SMEM) continue;
+            const int ctas = (int)std::min<uint64_t>(sm_threads / nt, (220 * 1024) / (smem + 1536));
+            if (ctas < 1) continue;
+            const double work = slots / (14.0 * n * nl * ns);
+            const double occ = std::min(1.0, ctas * nt / (double)sm_threads);
+            const double seg = mode == MODE_LANE ? (nl * esz >= 128 ? 1.0 : nl * esz >= 64 ? 1.15 : 1.6) : 1.0;
+            // (few lines: enough tiles for every SM)
+            const double tiles = std::ceil((double)nlines / nl);
+            const double idle = tiles < nsm ? std::min(4.0, nsm / tiles) : 1.0;
+            const double score = work * seg * idle / (0.3 + 0.7 * occ);
+            if (score < best) {
+                best = score;
+                x.nl = nl;
+                x.lsh = (uint32_t)ilog2(nl);
+                x.buf = (uint32_t)buf;
+                x.inplace = one;
+                *nt_out = nt;
+                *smem_out = (uint32_t)smem;
+            }
+        }
+    }
+    return best < 1e30;
+}
+
+static bool mix_ok(const rk_fft_desc& d, const PassSpec& p) {
+    int r[MIX_STAGES];
+    if (!lean_allowed(d) || !mix_radices(p.L, r)) return false;
+    const int dbl = d.dtype == RK_FMT_C128;
+    PassParams a;
+    LeanSide s;
+    MixPlan x;
+    uint32_t nt, sm;
+    pass_params(d, p, dbl, a);
+    return a.nlines < (int64_t(1) << 31) && lean_side(a.ld, a, dbl, p.L, p.mode == MODE_POS, 0, &s) && s.shift == 0 &&
+           lean_side(a.st, a, dbl, p.L, p.mode == MODE_POS, 0, &s) && mix_tile(p.L, dbl, p.mode, a.nlines, 148, x, &nt, &sm);
+}
+
+// A mixed-radix pass; `mem` allocates device memory that lives with the plan.
+template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int order, Alloc&& mem) {
+    const PassParams& p = r.prm;
+    auto lp = std::make_shared<LeanPass>();
+    LeanParams& q = lp->prm;
+    q = LeanParams{};
+    MixPlan x;
+    if (!lean_side(p.ld, p, dbl, r.L, r.mode == MODE_POS, 0, &q.ld) || !lean_side(p.st, p, dbl, r.L, r.mode == MODE_POS, 0, &q.st) ||
+        !mix_tile(r.L, dbl, r.mode, p.nlines, nsm, x, &q.mix_nt, &q.mix_smem)) {
+        set_error("no mixed-radix plan for this pass");
+        return RK_ERR_UNSUPPORTED;
+    }
+    const int esz = dbl ? 16 : 8;
+    const MixStage& last = x.stage[x.ns - 1];
+    void *tw = nullptr, *plan = nullptr;
+    int rc;
+    if ((rc = mem((int64_t)std::max<uint32_t>(last.tw, 1) * esz, &tw)) || (rc = mem(sizeof(MixPlan), &plan))) return rc;
+    for (int s = 0; s + 1 < x.ns; ++s) {
+        const MixStage& g = x.stage[s];
+        const int n = (int)((g.R - 1) * g.J);
+        k_gen_stage<<<(n + 255) / 256, 256>>>(dbl ? nullptr : (float2*)tw + g.tw, dbl ? (double2*)tw + g.tw : nullptr,
+                                              (int)(x.n / g.P), (int)g.R, (int)g.J);
+    }
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(plan, &x, sizeof(x), cudaMemcpyHostToDevice));
+    if (dbl) lean_mix_info_f64(r.mode, &lp->info);
+    else lean_mix_info_f32(r.mode, &lp->info);
+    CK(lp->info.prepare());
+    q.tw = tw;
+    q.mix = (const MixPlan*)plan;
+    q.mix_nl = x.nl;
+    q.nlines = (uint32_t)p.nlines;
+    q.rev = order & 1;
+    r.lean = lp;
+    return RK_OK;
 }
 
 // The row and column passes a plane pass splits into, with buffer `mid` between.
@@ -1802,7 +1971,9 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             int64_t blue_n = 0;
             for (const BlueAxis& ba : P.blue)
                 if (ba.axis == ps.axis) blue_n = ba.N;
-            if (lean_allowed(*desc)) {
+            if (ps.mixed) {
+                if ((rc = setup_mix(r, dbl, nsm, order++, alloc))) return fail(rc);
+            } else if (lean_allowed(*desc)) {
                 rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs, order);
                 if (rc) return fail(rc);
                 if (r.lean && ps.note != "bluestein-B1") ++order;   // (B1 and A2 are one launch)

@@ -269,3 +269,45 @@ def test_plane_as_rows_and_columns(rng, cuda, dtype, shape, shift):
             assert rel_l2(_run(src, out, axes, inverse, connect=connect if shift else None), ref) < fft_bound(dtype, shape[axes[0]] * shape[axes[1]])
         same = t.clone()
         assert rel_l2(_run(same, same, axes, inverse, connect=connect if shift else None), ref) < fft_bound(dtype, shape[axes[0]] * shape[axes[1]])
+
+
+MIXED = [6, 10, 12, 14, 15, 18, 21, 22, 24, 26, 33, 35, 36, 39, 45, 48, 49, 55, 60, 65, 66, 77, 78, 90, 91, 96, 99, 100, 104, 105, 110, 112,
+         117, 121, 130, 132, 143, 144, 154, 156, 169, 180, 182, 195, 196, 210, 225, 240, 243, 286, 343, 360, 385, 500, 625, 720, 729, 1000,
+         1001, 1080, 1155, 1331, 1536, 1920, 2197, 2401, 3000, 3003, 3072, 4000, 4095, 5000, 6000, 6561, 7350, 8000, 8085, 8190]
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("form", ["rows", "columns"])
+@pytest.mark.parametrize("n", MIXED)
+def test_mixed_radix_lines(rng, cuda, dtype, form, n):
+    """Every radix, two to four stages, whole and partial tiles; out of place, in place and
+    with the output shifted by half an odd or even length."""
+    import torch
+
+    from reikna_b200 import transformations as tr
+
+    rows = 1 if n > 4000 else 3 if n > 700 else 67
+    shape, axes = ((rows, n), (1,)) if form == "rows" else ((2, n, 5 if n > 700 else 21), (1,))
+    x = normal_array(rng, shape, dtype)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), axes, inverse), x, axes, inverse)
+
+    def connect(comp, out):
+        sh = tr.fftshift(out, axes=axes)
+        comp.parameter.output.connect(sh, sh.input, shifted=sh.output)
+
+    got = _run(t, torch.empty_like(t), axes, connect=connect)
+    ref = numpy.fft.fftshift(numpy.fft.fftn(x.astype(numpy.complex128), axes=axes), axes=axes)
+    assert rel_l2(got, ref) < fft_bound(dtype, n)
+    _check(_run(t, t, axes), x, axes)
+
+
+def test_mixed_radix_is_chosen_for_small_factors():
+    from reikna_b200 import _native as N
+
+    for n, note in ((1000, "mixed"), (97, "bluestein-fused"), (7350, "mixed"), (2 * 17, "bluestein-fused"), (1024, "single")):
+        assert N.describe(N.desc(N.FMT_C64, (5, n), (1,)))["passes"][0]["note"] == note
+        if note == "mixed":
+            assert N.describe(N.desc(N.FMT_C64, (5, n), (1,), N.FLAG_BATCHABLE))["passes"][0]["note"] == "bluestein-fused"
