@@ -165,8 +165,12 @@ int device_tables(int device, DeviceTables** out) {
         }
         total += li.tw_elems;
     }
-    CK(cudaMalloc(&t->lean_f, std::max<int64_t>(lnf, 1) * sizeof(float2)));
-    CK(cudaMalloc(&t->lean_d, std::max<int64_t>(lnd, 1) * sizeof(double2)));
+    // one block of whole 2 MiB granules: as small allocations of their own they filled the
+    // granule the plans' tables are cut from, and every plan then paid for mapping and
+    // unmapping one (1000 x 3001: 530 us to make and 330 us to drop, 140 and 17 otherwise)
+    const int64_t lean_bytes = lnd * sizeof(double2) + lnf * sizeof(float2), granule = int64_t(2) << 20;
+    CK(cudaMalloc(&t->lean_d, (lean_bytes + granule - 1) / granule * granule));
+    t->lean_f = (double2*)t->lean_d + lnd;
     t->bytes = (nf + lnf) * 8 + (ndd + lnd) * 16 + TW4_HALF * 48;
     for (const StageSeg& s : lsf) {
         const int n = (s.R - 1) * s.J;
