@@ -103,6 +103,9 @@ extern "C" {
 #define RK_FLAG_BATCHABLE 2048 /* plan only passes the persistent batched kernel has tile bodies for
                                 (no plane pass, strided fused Bluestein lines of at most 1024
                                 points); rk_batch_create members */
+#define RK_FLAG_REAL_ANY 8192  /* with RK_FLAG_REAL_POST / RK_FLAG_REAL_PRE: also lengths that are not
+                                powers of two, where one mixed-radix or Bluestein pass holds a
+                                line (contiguous complex edges below 4 GB) */
 #define RK_FLAG_BLUE_PAIR 4096 /* 8192-point complex64 fused Bluestein lines on a two-CTA
                                 cluster a line (each CTA one half of the padded spectrum, one
                                 exchange through distributed shared memory) instead of one CTA;

@@ -207,13 +207,14 @@ def array_pointer(arr, annotation) -> int:
     return int(arr.data_ptr())
 
 
-def _direct_call(names, plan, out_check, in_check, out_name, in_name, inverse):
+def _direct_call(names, plan, out_check, in_check, out_name, in_name, inverse, out_align=1, in_align=1):
     """The common call (positional arguments, one array each way, no scalars but the
     direction) without the dictionary, the numpy scalar and the pointer arrays of the
     general path: 7.7 -> 4.0 us a call of a one-kernel plan.  Returns False, before anything
     is queued, for any other call and for arrays that do not match; the general path then
     binds and checks it.  ``inverse``: the direction of computations without that
-    parameter, None to take it from the call."""
+    parameter, None to take it from the call; ``out_align`` / ``in_align``: boundaries (in
+    bytes) the arrays must start on."""
     import torch
 
     total = len(names)
@@ -249,7 +250,10 @@ def _direct_call(names, plan, out_check, in_check, out_name, in_name, inverse):
             stream = raw(device())
         elif type(stream) is not int:
             stream = stream_handle(stream)
-        plan.call(out.data_ptr(), inp.data_ptr(), inv, stream)
+        po, pi = out.data_ptr(), inp.data_ptr()
+        if po % out_align or pi % in_align:
+            return False
+        plan.call(po, pi, inv, stream)
         return True
 
     return call

@@ -43,6 +43,7 @@ struct MixPlan {
     uint32_t buf, pitch;   // elements of a buffer and of a line in it
     uint32_t pad;          // one pad word for each R0 positions (r0 divides by R0)
     uint32_t inplace;      // a thread has at most one butterfly a stage
+    uint32_t bufs;         // buffers: one in place, or with nothing between first and last stage
     FastDiv r0;
     MixStage stage[MIX_STAGES];
 };
@@ -115,9 +116,9 @@ struct LeanPass {
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
 };
 
-// Mixed-radix passes: the kernel of a mode
-void lean_mix_info_f32(int mode, LeanInfo* out);
-void lean_mix_info_f64(int mode, LeanInfo* out);
+// Mixed-radix passes: the kernel of a mode; real (contiguous lines): 1 RFFT, 2 IRFFT
+void lean_mix_info_f32(int mode, int real, LeanInfo* out);
+void lean_mix_info_f64(int mode, int real, LeanInfo* out);
 
 // A plan's launches of one direction, but for the user's pointers
 struct LeanChain {
@@ -134,7 +135,8 @@ struct LeanChain {
 // var 0 or 2 (transposed store); tw4: with four-step twiddles
 bool lean_info_f32(int L, int mode, int var, bool tw4, LeanInfo* out);
 bool lean_info_f64(int L, int mode, int var, bool tw4, LeanInfo* out);
-// Bluestein bodies: var 1 whole lines, 3 rows and 4 / 5 first / last columns (strided
+// Bluestein bodies: var 1 whole lines (6 / 7: contiguous ones with the real-spectrum step
+// after / before, RFFT and IRFFT), 3 rows and 4 / 5 first / last columns (strided
 // lines) of the three-pass form
 bool lean_blue_info_f32(int L, int mode, int var, LeanInfo* out);
 bool lean_blue_info_f64(int L, int mode, int var, LeanInfo* out);

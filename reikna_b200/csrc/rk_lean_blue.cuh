@@ -149,7 +149,70 @@ __device__ __forceinline__ void blue_core(const LeanParams& p, const cplx<T>* kp
     E::run(v, sm, ln, tb, tw);
 }
 
-template <typename T, int L, int MODE>
+// The real-spectrum step of a line (RFFT): outputs chirp[a] conj(v) to shared memory, then
+// bins in pairs k, N - k.
+template <typename T, class E>
+__device__ __forceinline__ void blue_bins_out(const LeanParams& p, uint32_t off, int ln, int tb, bool ok, cplx<T>* sm, cplx<T>* v) {
+    using V = cplx<T>;
+    using C = typename E::C;
+    const V* ch = reinterpret_cast<const V*>(p.chirp);
+    const int n = (int)p.blue_n;
+    V* z = sm + ln * C::LS;
+    lean_sync<C::WARP>();
+#pragma unroll
+    for (int i = 0; i < E::RT; ++i)
+        if (i % E::RL < E::RL / 2 && tb + E::ok(i) < n) z[tb + E::ok(i)] = cmulc(ch[tb + E::ok(i)], v[i]);
+    lean_sync<C::WARP>();
+    if (!ok) return;
+    const V* wk = reinterpret_cast<const V*>(p.rmix);
+    V* out = reinterpret_cast<V*>(p.st.base + off);
+#pragma unroll 1
+    for (int k = tb; 2 * k <= n; k += E::TPL) {
+        V o[2];
+        real_pair<T>(z[k], z[k == 0 ? 0 : n - k], __ldg(wk + k), T(0.5), o[0], o[1]);
+        if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
+        if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
+        out[k] = o[0];
+        if (k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * k < n) out[n - k] = o[1];
+    }
+}
+
+// The inverse step (IRFFT): bins to the half-length spectrum in shared memory, then times
+// the chirp into v.
+template <typename T, class E>
+__device__ __forceinline__ void blue_bins_in(const LeanParams& p, uint32_t off, int ln, int tb, cplx<T>* sm, cplx<T>* v) {
+    using V = cplx<T>;
+    using C = typename E::C;
+    const V* ch = reinterpret_cast<const V*>(p.chirp);
+    const V* wk = reinterpret_cast<const V*>(p.rmix);
+    const int n = (int)p.blue_n;
+    const V* in = reinterpret_cast<const V*>(p.ld.base + off);
+    V* z = sm + ln * C::LS;
+#pragma unroll 2
+    for (int k = tb; 2 * k <= n; k += E::TPL) {
+        V y[2] = {in[k], in[n - k]}, a, b;
+        if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, y);
+        if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(y);
+        if (k == 0) {
+            // bins 0 and N of a real signal are real
+            y[0].y = T(0);
+            y[1].y = T(0);
+        }
+        real_pair<T>(y[0], y[1], __ldg(wk + k), T(0.5), a, b);
+        z[k] = a;
+        if (k > 0 && 2 * k < n) z[n - k] = b;
+    }
+    lean_sync<C::WARP>();
+#pragma unroll
+    for (int i = 0; i < E::RT; ++i)
+        if (i % E::R0 < E::R0 / 2) {
+            const int a = tb + E::ik(i);
+            v[i] = a < n ? cmul(z[a], ch[a]) : cmk<V>(T(0), T(0));
+        }
+    lean_sync<C::WARP>();
+}
+
+template <typename T, int L, int MODE, int REAL>
 __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, MODE, 1>::MINB))
     k_lean_blue(const __grid_constant__ LeanParams p) {
     using V = cplx<T>;
@@ -163,9 +226,11 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE, 1>::NT), (LeanCfg<T, L, M
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
     const uint32_t lt = lean_tile(p) * NL + ln, line = min(lt, p.nlines - 1);
     V v[E::RT];
-    blue_load<T, E, MODE == MODE_POS>(p, lean_offset(p.ld, line), tb, 0, v);
+    if constexpr (REAL == 2) blue_bins_in<T, E>(p, lean_offset(p.ld, line), ln, tb, sm, v);
+    else blue_load<T, E, MODE == MODE_POS>(p, lean_offset(p.ld, line), tb, 0, v);
     blue_core<T, E, true>(p, reinterpret_cast<const V*>(p.blue_k), v, sm, ln, tb);
-    blue_store<T, E, MODE == MODE_POS>(p, lean_offset(p.st, line), tb, 0, lt < p.nlines, v);
+    if constexpr (REAL == 1) blue_bins_out<T, E>(p, lean_offset(p.st, line), ln, tb, lt < p.nlines, sm, v);
+    else blue_store<T, E, MODE == MODE_POS>(p, lean_offset(p.st, line), tb, 0, lt < p.nlines, v);
 }
 
 // Rows of the three-pass form: line (o, c, i) of N2 = L points; K and the twiddles of row c.
@@ -218,11 +283,12 @@ __global__ void __launch_bounds__((LeanCfg<T, L, MODE_LANE, 0>::NT), (LeanCfg<T,
     }
 }
 
-// VAR 1: whole lines; 3: rows of the three-pass form; 4 / 5: its first / last columns
+// VAR 1: whole lines (6 / 7: with the real-spectrum step after / before); 3: rows of the
+// three-pass form; 4 / 5: its first / last columns
 template <typename T, int L, int MODE, int VAR> struct LeanBlueLauncher {
-    using C = LeanCfg<T, L, MODE, (VAR >= 4 ? 0 : 1)>;
+    using C = LeanCfg<T, L, MODE, (VAR == 4 || VAR == 5 ? 0 : 1)>;
     static constexpr auto kernel() {
-        if constexpr (VAR == 1) return &k_lean_blue<T, L, MODE>;
+        if constexpr (VAR == 1 || VAR >= 6) return &k_lean_blue<T, L, MODE, (VAR >= 6 ? VAR - 5 : 0)>;
         else if constexpr (VAR == 3) return &k_lean_mid<T, L, MODE>;
         else return &k_lean_cols<T, L, VAR == 5>;
     }

@@ -6,6 +6,8 @@ namespace rk {
 #define RK_LB(LL, MODE, VAR) \
     if (L == LL && mode == MODE && var == VAR) { *out = LeanBlueLauncher<float, LL, MODE, VAR>::info(); return true; }
 
+bool lean_blue_real_info_f32(int L, int mode, int var, LeanInfo* out);
+
 bool lean_blue_info_f32(int L, int mode, int var, LeanInfo* out) {
     RK_LB(16, MODE_POS, 1) RK_LB(32, MODE_POS, 1) RK_LB(64, MODE_POS, 1) RK_LB(128, MODE_POS, 1)
     RK_LB(256, MODE_POS, 1) RK_LB(512, MODE_POS, 1) RK_LB(1024, MODE_POS, 1) RK_LB(2048, MODE_POS, 1)
@@ -20,7 +22,7 @@ bool lean_blue_info_f32(int L, int mode, int var, LeanInfo* out) {
     RK_LB(512, MODE_LANE, 4) RK_LB(1024, MODE_LANE, 4)
     RK_LB(32, MODE_LANE, 5) RK_LB(64, MODE_LANE, 5) RK_LB(128, MODE_LANE, 5) RK_LB(256, MODE_LANE, 5)
     RK_LB(512, MODE_LANE, 5) RK_LB(1024, MODE_LANE, 5)
-    return false;
+    return var >= 6 && lean_blue_real_info_f32(L, mode, var, out);
 }
 
 }  // namespace rk

@@ -146,18 +146,23 @@ template <typename T> struct MixCfg {
     static constexpr int NT = sizeof(T) == 4 ? 384 : 256, MINB = 2;
 };
 
-// One stage of radix R over the tile's butterflies.  FIRST reads the lines from global
-// memory, LAST writes them there; between, buffer `src` to buffer `dst`.
-template <typename T, int R, int MODE, bool FIRST, bool LAST>
+// Where a stage reads from and writes to: global memory (first stage, last stage), the
+// tile's buffers, or the tile's buffers at both ends of a real transform (first stage from
+// lines without pads, last stage to whole lines, before the real-spectrum step).
+enum MixEnd { MIX_GLOBAL, MIX_TILE, MIX_LINES };
+
+// One stage of radix R over the tile's butterflies.
+template <typename T, int R, int MODE, int SRC, int DST>
 __device__ __forceinline__ void mix_stage(const LeanParams& p, const MixPlan& x, const MixStage& g, const cplx<T>* src,
                                           cplx<T>* dst, const uint32_t* off_ld, const uint32_t* off_st, uint32_t valid) {
     using V = cplx<T>;
+    constexpr bool FIRST = SRC != MIX_TILE, LAST = DST != MIX_TILE;
     const uint32_t nb = g.nb, total = nb * x.nl, nll = x.nl;
     const V* tw = reinterpret_cast<const V*>(p.tw) + g.tw;
     auto pad = [&](uint32_t at) { return x.pad ? fd_div(x.r0, at) : 0u; };
     // distance between a butterfly's inputs and between its outputs
     const uint32_t rd = FIRST ? nb : MODE == MODE_LANE ? nb * nll : nb + pad(nb);
-    const uint32_t wr = LAST ? g.P : MODE == MODE_LANE ? g.P * nll : FIRST ? 1 : g.P + pad(g.P);
+    const uint32_t wr = DST == MIX_GLOBAL ? g.P : MODE == MODE_LANE ? g.P * nll : FIRST ? 1 : g.P + pad(g.P);
     uint32_t i = threadIdx.x;
     do {
         const bool act = i < total;
@@ -171,7 +176,11 @@ __device__ __forceinline__ void mix_stage(const LeanParams& p, const MixPlan& x,
         }
         V v[R];
         if (act) {
-            if constexpr (FIRST) {
+            if constexpr (SRC == MIX_LINES) {
+                const V* q = src + ln * x.n + b;
+#pragma unroll
+                for (int m = 0; m < R; ++m) v[m] = q[m * nb];
+            } else if constexpr (FIRST) {
                 if constexpr (MODE == MODE_POS) {
                     const V* lp = reinterpret_cast<const V*>(p.ld.base + off_ld[ln]) + b;
 #pragma unroll
@@ -192,15 +201,15 @@ __device__ __forceinline__ void mix_stage(const LeanParams& p, const MixPlan& x,
         }
         // P = L / R in the last stage: j1 = 0, output m at b + P m
         const uint32_t j1 = FIRST ? b : LAST ? 0 : fd_div(g.pdiv, b), l = FIRST ? 0 : b - j1 * g.P;
-        if constexpr (!LAST) {
-            if (act) {
+        if constexpr (DST != MIX_GLOBAL) {
+            if (!LAST && act) {
 #pragma unroll
                 for (int m = 1; m < R; ++m) v[m] = cmul(v[m], __ldg(tw + ((m - 1) * g.J + j1)));
             }
             // in place: every butterfly of the stage is in registers before one is written
-            if (!FIRST && x.inplace) __syncthreads();
+            if (SRC != MIX_GLOBAL && x.inplace) __syncthreads();
             if (act) {
-                const uint32_t at = l + g.P * R * j1;
+                const uint32_t at = LAST ? b : l + g.P * R * j1;
                 V* q = dst + (MODE == MODE_LANE ? at * nll + ln : ln * x.pitch + at + pad(at));
 #pragma unroll
                 for (int m = 0; m < R; ++m) q[m * wr] = v[m];
@@ -231,12 +240,12 @@ __device__ __forceinline__ void mix_stage(const LeanParams& p, const MixPlan& x,
     } while (i < total);
 }
 
-template <typename T, int MODE, bool FIRST, bool LAST>
+template <typename T, int MODE, int SRC, int DST>
 __device__ __forceinline__ void mix_radix(const LeanParams& p, const MixPlan& x, int s, const cplx<T>* src, cplx<T>* dst,
                                           const uint32_t* off_ld, const uint32_t* off_st, uint32_t valid) {
     const MixStage& g = x.stage[s];
 #define RK_MIX(R) \
-    case R: mix_stage<T, R, MODE, FIRST, LAST>(p, x, g, src, dst, off_ld, off_st, valid); break;
+    case R: mix_stage<T, R, MODE, SRC, DST>(p, x, g, src, dst, off_ld, off_st, valid); break;
     switch (g.R) {
         RK_MIX(2) RK_MIX(3) RK_MIX(4) RK_MIX(5) RK_MIX(6) RK_MIX(7) RK_MIX(8) RK_MIX(9)
         RK_MIX(10) RK_MIX(11) RK_MIX(12) RK_MIX(14) RK_MIX(15) RK_MIX(16)
@@ -244,7 +253,58 @@ __device__ __forceinline__ void mix_radix(const LeanParams& p, const MixPlan& x,
 #undef RK_MIX
 }
 
-template <typename T, int MODE>
+// The real-spectrum step of the tile's lines: z (pitch and pads of the tile) to bins
+// X[0 .. n) and, where stored, X[n].  w_k = exp(-i pi k / n) in rmix.
+template <typename T>
+__device__ __forceinline__ void mix_bins_out(const LeanParams& p, const MixPlan& x, const cplx<T>* z, const uint32_t* off_st,
+                                             uint32_t valid) {
+    using V = cplx<T>;
+    const V* wk = reinterpret_cast<const V*>(p.rmix);
+    const uint32_t n = x.n, pairs = n / 2 + 1;
+    auto at = [&](uint32_t k) { return k + (x.pad ? fd_div(x.r0, k) : 0u); };
+    for (uint32_t ln = 0; ln < valid; ++ln) {
+        const V* zl = z + ln * x.pitch;
+        V* out = reinterpret_cast<V*>(p.st.base + off_st[ln]);
+        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) {
+            V o[2];
+            real_pair<T>(zl[at(k)], zl[at(k == 0 ? 0 : n - k)], __ldg(wk + k), T(0.5), o[0], o[1]);
+            if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
+            if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
+            out[k] = o[0];
+            if (k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * k < n) out[n - k] = o[1];
+        }
+    }
+}
+
+// The inverse step: bins of the tile's lines to the half-length spectrum, lines of n points.
+template <typename T>
+__device__ __forceinline__ void mix_bins_in(const LeanParams& p, const MixPlan& x, cplx<T>* z, const uint32_t* off_ld) {
+    using V = cplx<T>;
+    const V* wk = reinterpret_cast<const V*>(p.rmix);
+    const uint32_t n = x.n, pairs = n / 2 + 1;
+    for (uint32_t ln = 0; ln < x.nl; ++ln) {
+        const V* in = reinterpret_cast<const V*>(p.ld.base + off_ld[ln]);
+        V* zl = z + ln * n;
+        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) {
+            V y[2] = {in[k], in[n - k]}, a, b;
+            if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, y);
+            if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(y);
+            if (k == 0) {
+                // bins 0 and n of a real signal are real
+                y[0].y = T(0);
+                y[1].y = T(0);
+            }
+            real_pair<T>(y[0], y[1], __ldg(wk + k), T(0.5), a, b);
+            zl[k] = a;
+            if (k > 0 && 2 * k < n) zl[n - k] = b;
+        }
+    }
+}
+
+// REAL 1: the real-spectrum step after the FFT (RFFT: sample pairs in, bins out); 2: the
+// inverse step before it (IRFFT).  The mirror of bin k is bin n - k of the same line, both
+// in shared memory.
+template <typename T, int MODE, int REAL>
 __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(const __grid_constant__ LeanParams p) {
     using V = cplx<T>;
     extern __shared__ __align__(16) unsigned char rk_smem[];
@@ -255,7 +315,7 @@ __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(con
     lean_begin();
     __syncthreads();
     V* buf0 = reinterpret_cast<V*>(rk_smem);
-    V* buf1 = x.inplace || x.ns < 3 ? buf0 : buf0 + x.buf;
+    V* buf1 = x.bufs == 1 ? buf0 : buf0 + x.buf;
     uint32_t* off_ld = reinterpret_cast<uint32_t*>(buf1 + x.buf);
     uint32_t* off_st = off_ld + x.nl;
     const uint32_t line0 = lean_tile(p) * x.nl;
@@ -266,29 +326,46 @@ __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(con
     }
     __syncthreads();
     const uint32_t valid = min(x.nl, p.nlines - line0);
-    mix_radix<T, MODE, true, false>(p, x, 0, nullptr, buf0, off_ld, off_st, valid);
-    // (not a loop: hoisting what its 15 bodies share out of it spilled 900 bytes a thread)
-    V* last = buf0;
+    if constexpr (REAL == 2) {
+        mix_bins_in<T>(p, x, buf0, off_ld);
+        __syncthreads();
+        mix_radix<T, MODE, MIX_LINES, MIX_TILE>(p, x, 0, buf0, buf1, off_ld, off_st, valid);
+        V* t = buf0;
+        buf0 = buf1;
+        buf1 = t;
+    } else {
+        mix_radix<T, MODE, MIX_GLOBAL, MIX_TILE>(p, x, 0, nullptr, buf0, off_ld, off_st, valid);
+    }
+    // (not a loop: hoisting what its bodies share out of it spilled 900 bytes a thread)
+    V *last = buf0, *other = buf1;
     if (x.ns > 2) {
         __syncthreads();
-        mix_radix<T, MODE, false, false>(p, x, 1, buf0, buf1, off_ld, off_st, valid);
+        mix_radix<T, MODE, MIX_TILE, MIX_TILE>(p, x, 1, buf0, buf1, off_ld, off_st, valid);
         last = buf1;
+        other = buf0;
     }
     if (x.ns > 3) {
         __syncthreads();
-        mix_radix<T, MODE, false, false>(p, x, 2, buf1, buf0, off_ld, off_st, valid);
+        mix_radix<T, MODE, MIX_TILE, MIX_TILE>(p, x, 2, buf1, buf0, off_ld, off_st, valid);
         last = buf0;
+        other = buf1;
     }
     __syncthreads();
-    mix_radix<T, MODE, false, true>(p, x, x.ns - 1, last, nullptr, off_ld, off_st, valid);
+    if constexpr (REAL == 1) {
+        mix_radix<T, MODE, MIX_TILE, MIX_LINES>(p, x, x.ns - 1, last, other, off_ld, off_st, valid);
+        __syncthreads();
+        mix_bins_out<T>(p, x, other, off_st, valid);
+    } else {
+        mix_radix<T, MODE, MIX_TILE, MIX_GLOBAL>(p, x, x.ns - 1, last, nullptr, off_ld, off_st, valid);
+    }
 }
 
-template <typename T, int MODE> struct LeanMixLauncher {
+template <typename T, int MODE, int REAL> struct LeanMixLauncher {
     static cudaError_t launch(const LeanParams& p, cudaStream_t st) {
-        return lean_launch(k_lean_mix<T, MODE>, (p.nlines + p.mix_nl - 1) / p.mix_nl, p.mix_nt, p.mix_smem, p, st);
+        return lean_launch(k_lean_mix<T, MODE, REAL>, (p.nlines + p.mix_nl - 1) / p.mix_nl, p.mix_nt, p.mix_smem, p, st);
     }
     static cudaError_t prepare() {
-        return cudaFuncSetAttribute(k_lean_mix<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
+        return cudaFuncSetAttribute(k_lean_mix<T, MODE, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
     }
 };
 

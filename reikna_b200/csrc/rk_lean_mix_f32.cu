@@ -3,10 +3,15 @@
 
 namespace rk {
 
-void lean_mix_info_f32(int mode, LeanInfo* out) {
+void lean_mix_info_f32(int mode, int real, LeanInfo* out) {
     *out = LeanInfo{};
-    out->launch = mode == MODE_POS ? &LeanMixLauncher<float, MODE_POS>::launch : &LeanMixLauncher<float, MODE_LANE>::launch;
-    out->prepare = mode == MODE_POS ? &LeanMixLauncher<float, MODE_POS>::prepare : &LeanMixLauncher<float, MODE_LANE>::prepare;
+#define RK_LM(MODE, REAL) \
+    if (mode == MODE && real == REAL) { \
+        out->launch = &LeanMixLauncher<float, MODE, REAL>::launch; \
+        out->prepare = &LeanMixLauncher<float, MODE, REAL>::prepare; \
+    }
+    RK_LM(MODE_POS, 0) RK_LM(MODE_LANE, 0) RK_LM(MODE_POS, 1) RK_LM(MODE_POS, 2)
+#undef RK_LM
 }
 
 }  // namespace rk

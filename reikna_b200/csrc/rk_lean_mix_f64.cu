@@ -3,10 +3,15 @@
 
 namespace rk {
 
-void lean_mix_info_f64(int mode, LeanInfo* out) {
+void lean_mix_info_f64(int mode, int real, LeanInfo* out) {
     *out = LeanInfo{};
-    out->launch = mode == MODE_POS ? &LeanMixLauncher<double, MODE_POS>::launch : &LeanMixLauncher<double, MODE_LANE>::launch;
-    out->prepare = mode == MODE_POS ? &LeanMixLauncher<double, MODE_POS>::prepare : &LeanMixLauncher<double, MODE_LANE>::prepare;
+#define RK_LM(MODE, REAL) \
+    if (mode == MODE && real == REAL) { \
+        out->launch = &LeanMixLauncher<double, MODE, REAL>::launch; \
+        out->prepare = &LeanMixLauncher<double, MODE, REAL>::prepare; \
+    }
+    RK_LM(MODE_POS, 0) RK_LM(MODE_LANE, 0) RK_LM(MODE_POS, 1) RK_LM(MODE_POS, 2)
+#undef RK_LM
 }
 
 }  // namespace rk

@@ -322,6 +322,7 @@ struct PassSpec {
     int64_t tw4_N = 0;
     int blue_axis = -1;     // fused Bluestein kernel spectrum owner
     int lean_var = 0;       // Bluestein body of the three-pass form (lean_blue_info), 0: none
+    int real = 0;           // lean pass with the real-spectrum step: 1 RFFT, 2 IRFFT
     bool mixed = false;     // mixed-radix pass of L points (rk_lean_mix.cuh)
     int mid = -1;           // a plane pass run as lean rows and columns: the buffer between
     bool pair = false;      // with the next pass: one plane-ordered pair launch
@@ -380,6 +381,7 @@ static bool lean_allowed(const rk_fft_desc& d);
 static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out);
 static int plane_mid(const rk_fft_desc& d, const PassSpec& p);
 static bool mix_ok(const rk_fft_desc& d, const PassSpec& p);
+static bool lean_blue_real_ok(const rk_fft_desc& d, const PassSpec& p);
 static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const PassSpec& last);
 
 static int plan_passes(const rk_fft_desc& d, Planned& P) {
@@ -407,6 +409,10 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
         set_error("a one-pass real transform takes no additive term, constant input or ignored output");
         return RK_ERR_UNSUPPORTED;
     }
+    // lengths other than powers of two: a whole-line mixed-radix or Bluestein pass with the
+    // real-spectrum step in it
+    const int real_any = !(d.flags & RK_FLAG_REAL_ANY) || !real_flags || (d.flags & RK_FLAG_ANTIPERIODIC) ? 0
+                         : (d.flags & RK_FLAG_REAL_POST) ? 1 : 2;
     int cur = SB_IN;
     auto array_out = [&](bool inplace_ok) -> int {
         if (inplace_ok && (cur == SB_T0 || cur == SB_T1)) return cur;
@@ -586,7 +592,8 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
                 p.st.buf = out; p.st.ax_len = n;
                 p.note = "mixed";
                 p.mixed = true;
-                if (!real_flags && !(d.flags & (RK_FLAG_R16 | RK_FLAG_BLUE_PAIR)) && mix_ok(d, p)) {
+                p.real = real_any;
+                if ((!real_flags || real_any) && !(d.flags & (RK_FLAG_R16 | RK_FLAG_BLUE_PAIR)) && mix_ok(d, p)) {
                     P.passes.push_back(p);
                     cur = out;
                     continue;
@@ -607,6 +614,7 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
             }
             if ((I == 1 && M <= PM) || (I > 1 && M <= blue_lane_max)) {
                 PassSpec p;
+                p.real = real_any;
                 p.L = (int)M; p.var = 1; p.blue_axis = ax;
                 p.mode = I == 1 ? MODE_POS : MODE_LANE;
                 // RK_FLAG_R16: 8192-point float32 lines on the 16-element plan with 512
@@ -703,7 +711,9 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
         const int64_t L = d.shape[ax];
         const bool bins_ok = ap ? spec.shape[ax] == L
                                 : (post ? (spec.shape[ax] == L || spec.shape[ax] == L + 1) : spec.shape[ax] == L + 1);
-        if (P.passes.size() != 1 || P.passes[0].var != (post ? 3 : 4) || spec.strides[ax] != 1 || !bins_ok ||
+        const bool one = P.passes.size() == 1 &&
+                         (P.passes[0].var == (post ? 3 : 4) || (P.passes[0].real && lean_blue_real_ok(d, P.passes[0])));
+        if (!one || spec.strides[ax] != 1 || !bins_ok ||
             spec.shift[ax] != 0 || (!post && d.output.shape[ax] != L)) {
             set_error(post ? "RK_FLAG_REAL_POST needs a one-pass transform of the last axis (a power of two of 8 to "
                              "8192 points, 4096 for complex128) with a contiguous output of L or L + 1 bins (L with "
@@ -968,7 +978,7 @@ static bool lean_allowed(const rk_fft_desc& d) {
 // store (var 2), whole-line Bluestein (var 1), or a body of the three-pass form.
 static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, const DeviceTables* tabs, int order) {
     const PassParams& p = r.prm;
-    const int bvar = ps.lean_var ? ps.lean_var : r.var == 1 ? 1 : 0;
+    const int bvar = ps.lean_var ? ps.lean_var : ps.real ? 5 + ps.real : r.var == 1 ? 1 : 0;
     const bool pos = r.mode == MODE_POS, tw4 = p.st.flags & SF_TW4;
     if (r.kind != PK_LINE || (r.var != 0 && r.var != 1 && r.var != 2)) return RK_OK;
     if (p.nlines >= (int64_t(1) << 31) || (p.ld.flags & SF_TW4)) return RK_OK;
@@ -986,10 +996,10 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
     } else if (!lean_info(dbl, r.L, r.mode, r.var, tw4, &lp->info)) {
         return RK_OK;
     }
-    if (!lean_side(p.ld, p, dbl, r.L, pos, bvar == 1 || bvar == 4 ? blue_n : 0, &q.ld)) return RK_OK;
-    if (!lean_side(p.st, p, dbl, r.L, pos && r.var != 2, bvar == 1 || bvar == 5 ? blue_n : 0, &q.st)) return RK_OK;
+    if (!lean_side(p.ld, p, dbl, r.L, pos, bvar == 1 || bvar == 4 || bvar >= 6 ? blue_n : 0, &q.ld)) return RK_OK;
+    if (!lean_side(p.st, p, dbl, r.L, pos && r.var != 2, bvar == 1 || bvar == 5 || bvar >= 6 ? blue_n : 0, &q.st)) return RK_OK;
     // (the strided first and last columns run the plain bodies' radix plans)
-    const int64_t off = tabs->lean_off[bvar == 1 || bvar == 3][dbl][r.mode][ilog2(r.L)];
+    const int64_t off = tabs->lean_off[bvar == 1 || bvar == 3 || bvar >= 6][dbl][r.mode][ilog2(r.L)];
     q.tw = dbl ? (const void*)((const double2*)tabs->lean_d + off) : (const void*)((const float2*)tabs->lean_f + off);
     q.tw4_hi = p.tw4_hi;
     q.tw4_lo = p.tw4_lo;
@@ -1108,7 +1118,7 @@ static int mix_radices(int64_t n, int* r) {
 // Tile of a mixed-radix pass: lines and threads a CTA, from the share of threads that hold
 // a butterfly in every stage, the CTAs an SM (registers: 768 complex64 threads, 512
 // complex128; shared memory) and, for strided lines, the width of their segments.
-static bool mix_tile(int64_t n, int dbl, int mode, int64_t nlines, int nsm, MixPlan& x, uint32_t* nt_out, uint32_t* smem_out) {
+static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int nsm, MixPlan& x, uint32_t* nt_out, uint32_t* smem_out) {
     int r[MIX_STAGES];
     const int ns = mix_radices(n, r);
     if (!ns) return false;
@@ -1145,7 +1155,8 @@ static bool mix_tile(int64_t n, int dbl, int mode, int64_t nlines, int nsm, MixP
                 one = one && rounds == 1;
             }
             const uint64_t buf = mode == MODE_LANE ? (uint64_t)n * nl : (uint64_t)x.pitch * nl;
-            const uint64_t smem = buf * esz * (one || ns < 3 ? 1 : 2) + nl * 8;
+            const uint32_t bufs = one || (ns < 3 && !real) ? 1 : 2;
+            const uint64_t smem = buf * esz * bufs + nl * 8;
             if (smem > MIX_SMEM) continue;
             const int ctas = (int)std::min<uint64_t>(sm_threads / nt, (220 * 1024) / (smem + 1536));
             if (ctas < 1) continue;
@@ -1162,6 +1173,7 @@ static bool mix_tile(int64_t n, int dbl, int mode, int64_t nlines, int nsm, MixP
                 x.lsh = (uint32_t)ilog2(nl);
                 x.buf = (uint32_t)buf;
                 x.inplace = one;
+                x.bufs = bufs;
                 *nt_out = nt;
                 *smem_out = (uint32_t)smem;
             }
@@ -1180,18 +1192,37 @@ static bool mix_ok(const rk_fft_desc& d, const PassSpec& p) {
     uint32_t nt, sm;
     pass_params(d, p, dbl, a);
     return a.nlines < (int64_t(1) << 31) && lean_side(a.ld, a, dbl, p.L, p.mode == MODE_POS, 0, &s) && s.shift == 0 &&
-           lean_side(a.st, a, dbl, p.L, p.mode == MODE_POS, 0, &s) && mix_tile(p.L, dbl, p.mode, a.nlines, 148, x, &nt, &sm);
+           lean_side(a.st, a, dbl, p.L, p.mode == MODE_POS, 0, &s) && mix_tile(p.L, dbl, p.mode, p.real, a.nlines, 148, x, &nt, &sm);
+}
+
+// Whether a whole-line pass with the real-spectrum step in it has a lean body.
+static bool lean_blue_real_ok(const rk_fft_desc& d, const PassSpec& p) {
+    LeanInfo li;
+    if (p.mixed) return true;   // (mix_ok looked)
+    return p.mode == MODE_POS && p.var == 1 && lean_blue_edges(d, p, p) &&
+           lean_blue_info(d.dtype == RK_FMT_C128, p.L, MODE_POS, 5 + p.real, &li);
+}
+
+// The table and flags of a real-spectrum step of n bins: w_k = exp(-i pi k / n).
+template <class Alloc> static int setup_real_step(LeanParams& q, int64_t n, bool nyquist, int dbl, Alloc&& mem) {
+    void* wt = nullptr;
+    if (const int rc = mem((n + 1) * (dbl ? 16 : 8), &wt)) return rc;
+    k_gen_rpost<<<(unsigned)((n + 256) / 256), 256>>>(n, dbl ? nullptr : (float2*)wt, dbl ? (double2*)wt : nullptr);
+    CK(cudaGetLastError());
+    q.rmix = wt;
+    q.rflags = nyquist ? LR_NYQ : 0;
+    return RK_OK;
 }
 
 // A mixed-radix pass; `mem` allocates device memory that lives with the plan.
-template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int order, Alloc&& mem) {
+template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int order, int real, bool nyquist, Alloc&& mem) {
     const PassParams& p = r.prm;
     auto lp = std::make_shared<LeanPass>();
     LeanParams& q = lp->prm;
     q = LeanParams{};
     MixPlan x;
     if (!lean_side(p.ld, p, dbl, r.L, r.mode == MODE_POS, 0, &q.ld) || !lean_side(p.st, p, dbl, r.L, r.mode == MODE_POS, 0, &q.st) ||
-        !mix_tile(r.L, dbl, r.mode, p.nlines, nsm, x, &q.mix_nt, &q.mix_smem)) {
+        !mix_tile(r.L, dbl, r.mode, real, p.nlines, nsm, x, &q.mix_nt, &q.mix_smem)) {
         set_error("no mixed-radix plan for this pass");
         return RK_ERR_UNSUPPORTED;
     }
@@ -1208,8 +1239,9 @@ template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int or
     }
     CK(cudaGetLastError());
     CK(cudaMemcpy(plan, &x, sizeof(x), cudaMemcpyHostToDevice));
-    if (dbl) lean_mix_info_f64(r.mode, &lp->info);
-    else lean_mix_info_f32(r.mode, &lp->info);
+    if (dbl) lean_mix_info_f64(r.mode, real, &lp->info);
+    else lean_mix_info_f32(r.mode, real, &lp->info);
+    if (real && (rc = setup_real_step(q, r.L, nyquist, dbl, mem))) return rc;
     CK(lp->info.prepare());
     q.tw = tw;
     q.mix = (const MixPlan*)plan;
@@ -1976,10 +2008,19 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             for (const BlueAxis& ba : P.blue)
                 if (ba.axis == ps.axis) blue_n = ba.N;
             if (ps.mixed) {
-                if ((rc = setup_mix(r, dbl, nsm, order++, alloc))) return fail(rc);
+                if ((rc = setup_mix(r, dbl, nsm, order++, ps.real, desc->output.shape[ps.axis] > ps.L, alloc))) return fail(rc);
             } else if (lean_allowed(*desc)) {
                 rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs, order);
                 if (rc) return fail(rc);
+                if (ps.real && r.lean) {
+                    auto lp = std::make_shared<LeanPass>(*r.lean);
+                    if ((rc = setup_real_step(lp->prm, blue_n, desc->output.shape[ps.axis] > blue_n, dbl, alloc))) return fail(rc);
+                    r.lean = lp;
+                }
+                if (ps.real && !r.lean) {
+                    set_error("no lean body for a real transform of this length");
+                    return fail(RK_ERR_UNSUPPORTED);
+                }
                 if (r.lean && ps.note != "bluestein-B1") ++order;   // (B1 and A2 are one launch)
             }
             bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);

@@ -143,6 +143,8 @@ def _fused_runner(fused, ann, esz: int, inverse: int, real_side: str):
 
     run.launches = fused.launches
     run.plan = fused
+    run.direct = (fused, ArrayCheck(ann["output"]), ArrayCheck(ann["input"]), "output", "input", inverse,
+                  esz if real_side == "output" else 1, esz if real_side == "input" else 1)
     return run
 
 
@@ -177,6 +179,9 @@ class RFFT(Computation):
             run.plan = route
             run.direct = (route, ArrayCheck(ann["output"]), ArrayCheck(ann["input"]), "output", "input", 0)
             return run
+        fused = _fused_plan(device, meta.shape[:-1], half, cdt, N.FLAG_REAL_POST | N.FLAG_REAL_ANY, half, half + store_last)
+        if fused is not None:
+            return _fused_runner(fused, ann, cdt.itemsize, 0, "input")
         h = _Half(device, meta.shape[:-1], half, cdt)
 
         def runner(stream: int, args):
@@ -208,7 +213,7 @@ class IRFFT(Computation):
         ann = _edges(self, "IRFFT")
         meta = self._meta
         half = meta.shape[-1] - 1
-        fused = _fused_plan(device, meta.shape[:-1], half, meta.dtype, N.FLAG_REAL_PRE, half + 1, half)
+        fused = _fused_plan(device, meta.shape[:-1], half, meta.dtype, N.FLAG_REAL_PRE | N.FLAG_REAL_ANY, half + 1, half)
         if fused is not None:
             return _fused_runner(fused, ann, meta.dtype.itemsize, 1, "output")
         h = _Half(device, meta.shape[:-1], half, meta.dtype)

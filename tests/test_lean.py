@@ -311,3 +311,56 @@ def test_mixed_radix_is_chosen_for_small_factors():
         assert N.describe(N.desc(N.FMT_C64, (5, n), (1,)))["passes"][0]["note"] == note
         if note == "mixed":
             assert N.describe(N.desc(N.FMT_C64, (5, n), (1,), N.FLAG_BATCHABLE))["passes"][0]["note"] == "bluestein-fused"
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.float32, numpy.float64])
+@pytest.mark.parametrize("half", [6, 9, 17, 30, 31, 33, 97, 100, 121, 255, 500, 513, 625, 1001, 1023, 1500, 2049, 3000, 4095, 4097, 6000, 8191, 8193])
+@pytest.mark.parametrize("rows", [1, 23])
+def test_real_lines_of_any_length(rng, cuda, dtype, half, rows):
+    """RFFT and IRFFT in one mixed-radix or Bluestein pass: even and odd half lengths, both
+    ends of the padded lengths, and the first lengths beyond (the multi-kernel route)."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import IRFFT, RFFT
+
+    n = 2 * half
+    x = rng.standard_normal((rows, n)).astype(dtype)
+    t = torch.from_numpy(x).to(cuda)
+    cdt = torch.complex64 if dtype == numpy.float32 else torch.complex128
+    bound = fft_bound(numpy.complex64 if dtype == numpy.float32 else numpy.complex128, n)
+    ref = numpy.fft.rfft(x.astype(numpy.float64), axis=1)
+    for last in (False, True):
+        out = torch.full((rows, half + (0 if last else 1)), float("nan"), dtype=cdt, device=cuda)
+        RFFT(ArrayMetadata((rows, n), dtype), dont_store_last=last).compile()(None, out, t)
+        torch.cuda.synchronize()
+        assert rel_l2(out.cpu().numpy(), ref[:, :out.shape[1]]) < bound
+    bins = ref.astype(numpy.complex64 if dtype == numpy.float32 else numpy.complex128)
+    bins[:, 0] += 3j   # ignored, as numpy does
+    bins[:, -1] -= 2j
+    spec = torch.from_numpy(bins).to(cuda)
+    back = torch.full((rows, n), float("nan"), dtype=t.dtype, device=cuda)
+    IRFFT(spec).compile()(None, back, spec)
+    torch.cuda.synchronize()
+    assert rel_l2(back.cpu().numpy(), numpy.fft.irfft(bins.astype(numpy.complex128), n=n, axis=1)) < bound
+
+
+@gpu
+def test_real_plans_of_any_length_take_scales(rng, cuda):
+    """Edge scales of one-pass real plans (through the C-ABI) in their bodies."""
+    import torch
+
+    from reikna_b200 import _native as N
+
+    for half in (500, 97):
+        c = 0.5 + 0.25j
+        x = torch.from_numpy(rng.standard_normal((5, 2 * half)).astype(numpy.float32)).to(cuda)
+        d = N.desc(N.FMT_C64, (5, half), (1,), N.FLAG_REAL_POST | N.FLAG_REAL_ANY)
+        d.input = N.edge(N.FMT_C64, (5, half))
+        d.output = N.edge(N.FMT_C64, (5, half + 1))
+        d.output.scale_re, d.output.scale_im = c.real, c.imag
+        out = torch.empty((5, half + 1), dtype=torch.complex64, device=cuda)
+        N.Plan(d).execute([out.data_ptr()], [x.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rel_l2(out.cpu().numpy(), numpy.fft.rfft(x.cpu().numpy().astype(numpy.float64)) * c) < fft_bound(numpy.complex64, 2 * half)
