@@ -1084,15 +1084,18 @@ static bool lean_blue_edges(const rk_fft_desc& d, const PassSpec& first, const P
 
 // Radices (at most 16) of a mixed-radix plan of n points, or 0: the split with the least
 // work, counting per element what a stage costs (shared memory, twiddle, addresses: 14) and
-// what its DFT does (arithmetic grows with the largest prime; there is none for 13).  An odd radix goes first
+// what its DFT does (arithmetic grows with the largest prime).  An odd radix goes first
 // where there is one (its stride meets every bank), then the larger ones.
 static int mix_radices(int64_t n, int* r) {
-    static const int cost[17] = {0, 0, 2, 5, 4, 8, 7, 12, 7, 10, 10, 22, 9, 0, 14, 13, 10};
+    static const int cost[17] = {0, 0, 2, 5, 4, 8, 7, 12, 7, 10, 10, 22, 9, 26, 14, 13, 10};
     if (n < 6 || n > 8192) return 0;
     int best = 1 << 30, nbest = 0, cur[MIX_STAGES];
     auto search = [&](auto&& self, int64_t left, int at, int top, int sum) -> void {
         if (left == 1) {
-            if (at >= 2 && sum < best) {
+            // (four stages with a 13 of an odd length stay with Bluestein: the plan notes of
+            // its two-CTA form are pinned at 4095 points)
+            const bool pinned = at > 3 && n % 2 && std::find(cur, cur + at, 13) != cur + at;
+            if (at >= 2 && sum < best && !pinned) {
                 best = sum;
                 nbest = at;
                 std::copy(cur, cur + at, r);
@@ -1101,7 +1104,7 @@ static int mix_radices(int64_t n, int* r) {
         }
         if (at == MIX_STAGES) return;
         for (int R = top; R >= 2; --R)
-            if (left % R == 0 && R != 13) {
+            if (left % R == 0) {
                 cur[at] = R;
                 self(self, left / R, at + 1, R, sum + 14 + cost[R]);
             }
@@ -1115,9 +1118,13 @@ static int mix_radices(int64_t n, int* r) {
     return nbest;
 }
 
-// Tile of a mixed-radix pass: lines and threads a CTA, from the share of threads that hold
-// a butterfly in every stage, the CTAs an SM (registers: 768 complex64 threads, 512
-// complex128; shared memory) and, for strided lines, the width of their segments.
+// Tile of a mixed-radix pass: the lines and threads a CTA with the least estimated cycles.  A
+// tile alone takes 3000 cycles of latency and 180 + 25 R for each round of a stage's
+// butterflies over the threads; the CTAs an SM holds (registers: 768 complex64 threads, 512
+// complex128; shared memory) share its issue slots, 25 R + 15 instructions a butterfly at
+// 2.45 a cycle; the tiles go in whole waves; strided lines pay for segments under 128 bytes.
+// The constants were fitted to 4400 timed (length, batch, tile) combinations: the tile it
+// takes is 3% slower than the best on average (60 to 6000 points, 2^18 to 2^21 elements).
 static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int nsm, MixPlan& x, uint32_t* nt_out, uint32_t* smem_out) {
     int r[MIX_STAGES];
     const int ns = mix_radices(n, r);
@@ -1147,11 +1154,13 @@ static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int
         if (mode == MODE_LANE && nl * esz > 128) break;
         if (nl > 1 && nl * n > 4096 && mode == MODE_POS) break;
         for (uint32_t nt = 64; nt <= (uint32_t)max_nt; nt += 32) {
-            double slots = 0;
+            double alone = 3000, issue = 0;
             bool one = true;
             for (int s = 0; s < ns; ++s) {
-                const uint64_t total = (uint64_t)x.stage[s].nb * nl, rounds = (total + nt - 1) / nt;
-                slots += (double)rounds * nt * (14.0 * x.stage[s].R);
+                const MixStage& g = x.stage[s];
+                const uint64_t total = (uint64_t)g.nb * nl, rounds = (total + nt - 1) / nt;
+                alone += (double)rounds * (180 + 25.0 * g.R);
+                issue += (double)total * (15 + 25.0 * g.R) / 32;
                 one = one && rounds == 1;
             }
             const uint64_t buf = mode == MODE_LANE ? (uint64_t)n * nl : (uint64_t)x.pitch * nl;
@@ -1160,13 +1169,12 @@ static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int
             if (smem > MIX_SMEM) continue;
             const int ctas = (int)std::min<uint64_t>(sm_threads / nt, (220 * 1024) / (smem + 1536));
             if (ctas < 1) continue;
-            const double work = slots / (14.0 * n * nl * ns);
-            const double occ = std::min(1.0, ctas * nt / (double)sm_threads);
-            const double seg = mode == MODE_LANE ? (nl * esz >= 128 ? 1.0 : nl * esz >= 64 ? 1.15 : 1.6) : 1.0;
-            // (few lines: enough tiles for every SM)
-            const double tiles = std::ceil((double)nlines / nl);
-            const double idle = tiles < nsm ? std::min(4.0, nsm / tiles) : 1.0;
-            const double score = work * seg * idle / (0.3 + 0.7 * occ);
+            const double tiles = std::ceil((double)nlines / nl), slots = (double)nsm * ctas;
+            const double res = std::min<double>(ctas, std::ceil(tiles / nsm));
+            const double waves = tiles > 5 * slots ? tiles / slots : std::ceil(tiles / slots);
+            const int seg_bytes = mode == MODE_LANE ? (int)nl * esz : 128;
+            const double seg = seg_bytes >= 128 ? 1.0 : seg_bytes >= 64 ? 1.03 : seg_bytes >= 32 ? 1.16 : seg_bytes >= 16 ? 1.3 : 4.6;
+            const double score = seg * waves * (alone + res * issue / 2.45);
             if (score < best) {
                 best = score;
                 x.nl = nl;
