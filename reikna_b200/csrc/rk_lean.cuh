@@ -80,7 +80,7 @@ RK_LP(double, 32, MODE_LANE, false, 8, 8, 4)
 RK_LP(double, 64, MODE_LANE, false, 8, 8, 8)
 RK_LP(double, 128, MODE_LANE, false, 16, 16, 8)
 RK_LP(double, 256, MODE_LANE, false, 16, 16, 16)
-RK_LP(double, 512, MODE_LANE, false, 8, 8, 8, 8)
+RK_LP(double, 512, MODE_LANE, false, 16, 16, 16, 2)
 // Bluestein passes (padded length M = L)
 RK_LP(float, 16, MODE_POS, true, 4, 4, 4)
 RK_LP(float, 32, MODE_POS, true, 8, 8, 4)
@@ -116,7 +116,7 @@ RK_LP(double, 32, MODE_LANE, true, 8, 8, 4)
 RK_LP(double, 64, MODE_LANE, true, 8, 8, 8)
 RK_LP(double, 128, MODE_LANE, true, 16, 16, 8)
 RK_LP(double, 256, MODE_LANE, true, 16, 16, 16)
-RK_LP(double, 512, MODE_LANE, true, 8, 8, 8, 8)
+RK_LP(double, 512, MODE_LANE, true, 16, 16, 2, 16)
 RK_LP(double, 1024, MODE_LANE, true, 16, 16, 4, 16)
 #undef RK_LP
 

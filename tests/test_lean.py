@@ -364,3 +364,50 @@ def test_real_plans_of_any_length_take_scales(rng, cuda):
         N.Plan(d).execute([out.data_ptr()], [x.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
         torch.cuda.synchronize()
         assert rel_l2(out.cpu().numpy(), numpy.fft.rfft(x.cpu().numpy().astype(numpy.float64)) * c) < fft_bound(numpy.complex64, 2 * half)
+
+
+@gpu
+def test_dependent_launches_in_graphs_and_streams(rng, cuda):
+    """Chains of early-placed launches behind copies, forks and joins, captured and not: each
+    result is that of the calls one by one."""
+    import torch
+
+    from reikna_b200.fft import FFT
+
+    src = torch.from_numpy(normal_array(rng, (24, 96, 250), numpy.complex64)).to(cuda)
+    a, b, c = torch.empty_like(src), torch.empty_like(src), torch.empty_like(src)
+    both, last = FFT(src, axes=(1, 2)).compile(), FFT(src, axes=(0,)).compile()
+    side = torch.cuda.Stream()
+
+    def chain():
+        a.copy_(src)
+        both(None, b, a, 0)              # rows, columns
+        fork = torch.cuda.Event()
+        fork.record()
+        side.wait_event(fork)
+        with torch.cuda.stream(side):
+            last(None, c, b, 0)          # reads b beside the next call's reads
+        both(None, a, b, 1)              # back to src
+        join = torch.cuda.Event()
+        join.record(side)
+        torch.cuda.current_stream().wait_event(join)
+        c.mul_(2.0)
+        b.zero_()
+
+    ref = 2 * numpy.fft.fftn(src.cpu().numpy().astype(numpy.complex128))
+    for _ in range(3):
+        chain()
+    torch.cuda.synchronize()
+    assert rel_l2(c.cpu().numpy(), ref) < fft_bound(numpy.complex64, src.numel())
+    assert rel_l2(a.cpu().numpy(), src.cpu().numpy()) < 2 * fft_bound(numpy.complex64, 96 * 250)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for scale in (1.0, 3.0):
+        src.mul_(scale)
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        ref = 2 * numpy.fft.fftn(src.cpu().numpy().astype(numpy.complex128))
+        assert rel_l2(c.cpu().numpy(), ref) < fft_bound(numpy.complex64, src.numel())
+        assert rel_l2(a.cpu().numpy(), src.cpu().numpy()) < 2 * fft_bound(numpy.complex64, 96 * 250)
