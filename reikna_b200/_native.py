@@ -385,10 +385,11 @@ class Plan:
 
     def profile_read(self) -> tuple[list[float], int]:
         """(summed ms per pass, number of recorded executions); synchronises."""
-        ms = (ctypes.c_double * max(1, self.launches))()
+        passes = self.launches_total
+        ms = (ctypes.c_double * max(1, passes))()
         calls = ctypes.c_int32(0)
-        check(lib().rk_fft_profile_read(self._h, ms, self.launches, ctypes.byref(calls)))
-        return list(ms[: self.launches]), int(calls.value)
+        check(lib().rk_fft_profile_read(self._h, ms, passes, ctypes.byref(calls)))
+        return list(ms[:passes]), int(calls.value)
 
     def describe(self) -> dict:
         return describe(self.desc)

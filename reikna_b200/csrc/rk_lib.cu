@@ -2151,7 +2151,12 @@ int rk_fft_plan_device_bytes(const rk_fft_plan* plan, int64_t* bytes) {
 
 int rk_fft_plan_launches(const rk_fft_plan* plan, int32_t* n) {
     if (!plan || !n) { set_error("null argument"); return RK_ERR_INVALID; }
-    *n = (int32_t)plan->passes.size();
+    *n = 0;
+    for (size_t i = 0; i < plan->passes.size(); ++i) {
+        const PassRec& r = plan->passes[i];
+        *n += r.lean && r.lean->second ? 2 : 1;   // a plane as rows and columns
+        if (r.pair_first || (r.lean && r.lean->fuse_next)) ++i;   // the next pass' work is done
+    }
     return RK_OK;
 }
 
