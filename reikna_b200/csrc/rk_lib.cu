@@ -487,7 +487,6 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
             p.st.buf = out; p.st.ax_len = p.L1; p.st.cA = 0; p.st.jB = 1;
             p.note = "plane";
             p.mid = plane_mid(d, p);
-            if (p.mid == SB_T0) P.need_T0 = true;
             P.passes.push_back(p);
             cur = out;
             axes.erase(axes.begin(), axes.begin() + 2);
@@ -1275,27 +1274,29 @@ static void plane_split(const rk_fft_desc& d, const PassSpec& p, int mid, PassSp
 }
 
 // Whether a plane pass runs as two lean line passes, rows then columns, and through which
-// buffer (the output itself where the columns can be transformed in place there, else a
-// temporary); -1: the clustered kernel.  Two passes over memory at 85 to 95% of the copy
-// rate beat one at 40% (its CTAs wait for their cluster's exchange): 256 x 256 x 256
-// complex64 planes 94.3 -> 85.7 us, 1024 x 128 x 128 85.3 -> 82.1, 16 x 256 x 256 12.3 -> 9.6.
-// Where the clustered kernel keeps more in flight (64 x 64 complex64: one CTA a plane;
-// 128 x 128 complex128) it stays for arrays that L2 does not hold: 4096 x 64 x 64 71.0
-// against 81.1 us, 512 x 128 x 128 80.0 against 86.2; below, the lean passes are as fast or
-// faster (1024 x 64 x 64 21.8 against 23.3).
+// buffer (the pass' own temporary, or the output where the columns can be transformed in
+// place there); -1: the clustered kernel.  While L2 holds the array the second pass costs
+// little and both run far closer to the copy rate than the cluster's exchange lets one pass:
+// 16 x 256 x 256 complex64 12.3 -> 9.6 us, 128 x 256 x 256 51.8 -> 45.1, 64 x 128 x 128 10.3 ->
+// 9.4.  Beyond 64 MB the extra round trip through HBM counts: 4096 x 64 x 64 complex64 71.0 us
+// clustered against 81.1, 512 x 128 x 128 complex128 80.0 against 86.2, and 256 x 256 x 256 in
+// steps over three streams 125 us a step against 138 (alone on one stream the line passes
+// win, 135 against 145); 128 x 128 complex64 planes take the line passes at every size
+// (1024 of them: 82.1 against 85.3).
 static int plane_mid(const rk_fft_desc& d, const PassSpec& p) {
     const int dbl = d.dtype == RK_FMT_C128;
     if (!lean_allowed(d) || (d.flags & RK_FLAG_PLANE_WIDE)) return -1;
     const int64_t bytes = p.O * p.L1 * p.L2 * (dbl ? 16 : 8);
-    if (bytes > (int64_t(64) << 20) && p.L1 == (dbl ? 128 : 64)) return -1;
+    if (bytes > (int64_t(64) << 20) && (p.L1 == (dbl ? 128 : 64) || p.L1 == 256)) return -1;
     std::vector<int> mids;
     if (p.st.buf != SB_OUT) {
         mids = {p.st.buf};
     } else {
         bool plain = true;
         for (int i = 0; i < d.ndim; ++i) plain = plain && d.output.shift[i] == 0;
+        // (a remapped output would need a temporary of the plan, which a plan of one pass
+        // does not have: it may run on several streams at once)
         if (plain) mids.push_back(SB_OUT);
-        mids.push_back(SB_T0);
     }
     for (int mid : mids) {
         PassSpec rows, cols;
@@ -1844,6 +1845,11 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
     for (int i = 0; i < desc->naxes; ++i) ntot *= desc->shape[desc->axes[i]];
     plan->n_total = (double)ntot;
     int order = 0;   // lean launches so far
+    // Strided passes after a clustered plane pass keep the persistent TMA-fed kernel: with
+    // transforms on several streams the lean kernel's stream of CTAs keeps clusters from
+    // finding 16 free slots at once (256^3 over three streams 138 us a step against 125;
+    // alone the lean pass takes 48 us against 51).
+    bool clustered = false;
     for (const PassSpec& ps : P.passes) {
         PassRec r;
         r.kind = ps.kind;
@@ -1966,6 +1972,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
         r.L1 = ps.L1;
         r.L2 = ps.L2;
         r.axis2 = ps.axis2;
+        if (ps.kind == PK_PLANE && ps.mid < 0 && ps.L1 > 64) clustered = true;
         if (ps.kind == PK_PLANE && ps.mid >= 0) {
             PassSpec half[2];
             plane_split(*desc, ps, ps.mid, half[0], half[1]);
@@ -2017,7 +2024,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
                 if (ba.axis == ps.axis) blue_n = ba.N;
             if (ps.mixed) {
                 if ((rc = setup_mix(r, dbl, nsm, order++, ps.real, desc->output.shape[ps.axis] > ps.L, alloc))) return fail(rc);
-            } else if (lean_allowed(*desc)) {
+            } else if (lean_allowed(*desc) && !(clustered && ps.mode == MODE_LANE)) {
                 rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs, order);
                 if (rc) return fail(rc);
                 if (ps.real && r.lean) {
