@@ -14,6 +14,7 @@
 #include <cooperative_groups.h>
 
 #include "rk_async.cuh"
+#include "rk_dependent.cuh"
 #include "rk_internal.h"
 #include "rk_kernels.cuh"
 
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(PlaneCfg<T, L1, L2, Q>::NT, (PlaneTmaCfg<T, L1
     // uses the same ones; loads from there do not wait on L2)
     for (int i = tid; i < TC::TW2; i += C::NT) tw[i] = reinterpret_cast<const V*>(p.tw)[i];
     for (int i = tid; i < TC::TW1; i += C::NT) tw2[i] = reinterpret_cast<const V*>(p.tw2)[i];
+    dependent_wait();
     const int q = Q > 1 ? (int)cg::this_cluster().block_rank() : 0;
     const int64_t ncl = gridDim.x / Q;
     const int ln = tid / ER::TPL, tb = tid % ER::TPL;
@@ -302,8 +304,9 @@ template <typename T, int L1, int L2, int Q> struct PlaneTmaLauncher {
         a[0].val.clusterDim.x = Q;
         a[0].val.clusterDim.y = 1;
         a[0].val.clusterDim.z = 1;
+        a[Q > 1 ? 1 : 0] = dependent_launch();
         cfg.attrs = a;
-        cfg.numAttrs = Q > 1 ? 1 : 0;
+        cfg.numAttrs = Q > 1 ? 2 : 1;
         return cfg;
     }
     // nblocks = CTAs of the persistent grid (a multiple of Q)
@@ -311,15 +314,16 @@ template <typename T, int L1, int L2, int Q> struct PlaneTmaLauncher {
         cudaError_t e = attr();
         if (e != cudaSuccess) return e;
         if (nblocks <= 0) return cudaSuccess;
-        cudaLaunchAttribute a[1];
+        cudaLaunchAttribute a[2];
         cudaLaunchConfig_t cfg = config(nblocks, st, a);
         return cudaLaunchKernelEx(&cfg, k_plane_tma<T, L1, L2, Q>, p);
     }
     // clusters that fit on the device at once
     static int clusters() {
         if (attr() != cudaSuccess) return 0;
-        cudaLaunchAttribute a[1];
+        cudaLaunchAttribute a[2];
         cudaLaunchConfig_t cfg = config(Q * 256, nullptr, a);
+        cfg.numAttrs = 1;
         int n = 0;
         if (Q > 1) {
             if (cudaOccupancyMaxActiveClusters(&n, k_plane_tma<T, L1, L2, Q>, &cfg) != cudaSuccess) return 0;

@@ -1,6 +1,7 @@
 // Persistent TMA-fed line pass (the kernel template; instantiated by rk_tma.cu).
 #pragma once
 #include "rk_async.cuh"
+#include "rk_dependent.cuh"
 #include "rk_internal.h"
 #include "rk_kernels.cuh"
 
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(TmaCfg<T, L, MODE>::NT) k_line_tma(const __gri
         for (int i = tid; i < C::TWN; i += C::NT) tws[i] = tw[i];
         tw = tws;   // made visible by the barrier after the mbarrier set-up
     }
+    dependent_wait();
     const int ln = MODE == MODE_POS ? tid / TPL : tid % NL;
     const int tb = MODE == MODE_POS ? tid % TPL : tid / NL;
 
@@ -133,8 +135,16 @@ template <typename T, int L, int MODE> struct TmaLauncher {
             attr_done = true;
         }
         if (nblocks <= 0) return cudaSuccess;
-        k_line_tma<T, L, MODE><<<(unsigned)nblocks, C::NT, C::SMEM, st>>>(p);
-        return cudaGetLastError();
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)nblocks, 1, 1);
+        cfg.blockDim = dim3(C::NT, 1, 1);
+        cfg.dynamicSmemBytes = C::SMEM;
+        cfg.stream = st;
+        cudaLaunchAttribute a[1];
+        a[0] = dependent_launch();
+        cfg.attrs = a;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_line_tma<T, L, MODE>, p);
     }
     static int per_sm() {
         int n = 0;
