@@ -120,6 +120,17 @@ RK_LP(double, 512, MODE_LANE, true, 16, 16, 2, 16)
 RK_LP(double, 1024, MODE_LANE, true, 16, 16, 4, 16)
 #undef RK_LP
 
+// Plan of a few complex128 lines' four-step first pass (VAR 8): 512-point columns on 8 elements
+// a thread, whose twice as many threads hide its chain of table twiddle loads while
+// they do not fill the GPU.  2^18 points, 8 against 16 elements: 1 line 14.7 us against 19.7, 2
+// 15.3 against 21.5, but 8 lines 48.6 against 46.9 and 64 328 against 285.
+template <typename T, int L, int MODE, int VAR> struct LeanPick {
+    using P = LeanPlan<T, L, MODE, VAR == 1>;
+};
+template <> struct LeanPick<double, 512, MODE_LANE, 8> {
+    using P = LeanRadix<8, 8, 8, 8>;
+};
+
 // stage twiddle table of a plan: [m - 1][j1] of stage s after the earlier stages'
 template <int L, class P> struct LeanTw {
     static constexpr int size_of(int s) {
@@ -137,9 +148,10 @@ template <int L, class P> struct LeanTw {
 
 // VAR 0: plain; 1: Bluestein bodies (rk_lean_blue.cuh: two FFTs of the line with the
 // kernel spectrum between); 2: contiguous lines stored lane-fastest (transposed) through
-// shared memory; 5: the same for magnitudes (rk_lean_real.cuh)
+// shared memory; 5: the same for magnitudes (rk_lean_real.cuh); 8: plain, a few lines'
+// four-step first pass (LeanPick)
 template <typename T, int L, int MODE, int VAR> struct LeanCfg {
-    using P = LeanPlan<T, L, MODE, VAR == 1>;
+    using P = typename LeanPick<T, L, MODE, VAR>::P;
     using V = cplx<T>;
     static constexpr int RT = P::RT, TPL = L / RT, ESZ = sizeof(V);
     static constexpr int SEG = 128 / ESZ;   // elements of a 128-byte segment

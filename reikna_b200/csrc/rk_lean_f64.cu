@@ -16,6 +16,7 @@ bool lean_info_f64(int L, int mode, int var, bool tw4, LeanInfo* out) {
     RK_LN(2, MODE_LANE, 0, false) RK_LN(4, MODE_LANE, 0, false) RK_LN(8, MODE_LANE, 0, false)
     RK_LN(16, MODE_LANE, 0, false)
     RK_LN_LANE(32) RK_LN_LANE(64) RK_LN_LANE(128) RK_LN_LANE(256) RK_LN_LANE(512)
+    RK_LN(512, MODE_LANE, 8, true)
     return false;
 }
 

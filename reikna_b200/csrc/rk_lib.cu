@@ -36,6 +36,7 @@ namespace rk {
 
 constexpr int ilog2_c(int n) { return n <= 1 ? 0 : 1 + ilog2_c(n / 2); }
 
+constexpr int LEAN_TW_SLOT = 15;   // table slot of LeanPick<double, 512, MODE_LANE, 8>'s plan
 static bool lean_blue_info(int dbl, int L, int mode, int var, LeanInfo* out) {
     return dbl ? lean_blue_info_f64(L, mode, var, out) : lean_blue_info_f32(L, mode, var, out);
 }
@@ -164,6 +165,19 @@ int device_tables(int device, DeviceTables** out) {
             (dbl ? lsd : lsf).push_back(g);
         }
         total += li.tw_elems;
+    }
+    // the plan of a few complex128 lines' first pass, in an unused slot
+    {
+        LeanInfo li;
+        std::vector<StageSeg> segs;
+        lean_info(1, 512, MODE_LANE, 8, true, &li);
+        li.segments(segs);
+        t->lean_off[0][1][MODE_LANE][LEAN_TW_SLOT] = lnd;
+        for (StageSeg g : segs) {
+            g.off += lnd;
+            lsd.push_back(g);
+        }
+        lnd += li.tw_elems;
     }
     // one block of whole 2 MiB granules: as small allocations of their own they filled the
     // granule the plans' tables are cut from, and every plan then paid for mapping and
@@ -982,6 +996,8 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
     if (r.kind != PK_LINE || (r.var != 0 && r.var != 1 && r.var != 2)) return RK_OK;
     if (p.nlines >= (int64_t(1) << 31) || (p.ld.flags & SF_TW4)) return RK_OK;
     auto lp = std::make_shared<LeanPass>();
+    // up to four lines of 2^18 points (measured at LeanPick)
+    const bool few = dbl && tw4 && !bvar && r.var == 0 && r.mode == MODE_LANE && r.L == 512 && p.nlines <= 2048;
     LeanParams& q = lp->prm;
     q = LeanParams{};
     if (bvar) {
@@ -992,13 +1008,13 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
         q.jB = (uint32_t)(bvar == 4 ? p.ld.jB : bvar == 5 ? p.st.jB : 1);
         q.chirp = bvar == 5 ? p.st.chirp : p.ld.chirp;
         q.blue_k = p.blue_k;
-    } else if (!lean_info(dbl, r.L, r.mode, r.var, tw4, &lp->info)) {
+    } else if (!lean_info(dbl, r.L, r.mode, few ? 8 : r.var, tw4, &lp->info)) {
         return RK_OK;
     }
     if (!lean_side(p.ld, p, dbl, r.L, pos, bvar == 1 || bvar == 4 || bvar >= 6 ? blue_n : 0, &q.ld)) return RK_OK;
     if (!lean_side(p.st, p, dbl, r.L, pos && r.var != 2, bvar == 1 || bvar == 5 || bvar >= 6 ? blue_n : 0, &q.st)) return RK_OK;
     // (the strided first and last columns run the plain bodies' radix plans)
-    const int64_t off = tabs->lean_off[bvar == 1 || bvar == 3 || bvar >= 6][dbl][r.mode][ilog2(r.L)];
+    const int64_t off = tabs->lean_off[bvar == 1 || bvar == 3 || bvar >= 6][dbl][r.mode][few ? LEAN_TW_SLOT : ilog2(r.L)];
     q.tw = dbl ? (const void*)((const double2*)tabs->lean_d + off) : (const void*)((const float2*)tabs->lean_f + off);
     q.tw4_hi = p.tw4_hi;
     q.tw4_lo = p.tw4_lo;

@@ -81,6 +81,19 @@ def test_two_pass_lines(rng, cuda, dtype, n, shape):
 
 
 @gpu
+@pytest.mark.parametrize("rows", [1, 4, 5])
+def test_few_two_pass_lines(rng, cuda, rows):
+    """complex128 lines of 2^18 points on both sides of the first pass's choice of plan."""
+    import torch
+
+    x = normal_array(rng, (rows, 2**18), numpy.complex128)
+    t = torch.from_numpy(x).to(cuda)
+    for inverse in (0, 1):
+        _check(_run(t, torch.empty_like(t), (1,), inverse), x, (1,), inverse)
+    _check(_run(t, t, (1,)), x, (1,))
+
+
+@gpu
 @pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
 @pytest.mark.parametrize("shape,axes", [((6, 64, 32), (0,)), ((5, 64, 33), (1,)), ((4, 5, 256), (2,)), ((16, 8, 7), (0, 1)),
                                         ((32, 32, 32), (0, 1, 2)), ((2, 3, 4, 5, 16), (1, 4))])
