@@ -1861,7 +1861,8 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
     for (int i = 0; i < desc->naxes; ++i) ntot *= desc->shape[desc->axes[i]];
     plan->n_total = (double)ntot;
     int order = 0;   // lean launches so far
-    // Strided passes after a clustered plane pass keep the persistent TMA-fed kernel: with
+    // Strided passes after a clustered plane pass keep the general kernels, the persistent
+    // TMA-fed one where it applies (but for Bluestein bodies only the lean ones have): with
     // transforms on several streams the lean kernel's stream of CTAs keeps clusters from
     // finding 16 free slots at once (256^3 over three streams 138 us a step against 125;
     // alone the lean pass takes 48 us against 51).
@@ -2038,9 +2039,11 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             int64_t blue_n = 0;
             for (const BlueAxis& ba : P.blue)
                 if (ba.axis == ps.axis) blue_n = ba.N;
+            const bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);
+            const bool lean_only = !ok || ps.lean_var;   // (no general kernel does this pass' work)
             if (ps.mixed) {
                 if ((rc = setup_mix(r, dbl, nsm, order++, ps.real, desc->output.shape[ps.axis] > ps.L, alloc))) return fail(rc);
-            } else if (lean_allowed(*desc) && !(clustered && ps.mode == MODE_LANE)) {
+            } else if (lean_allowed(*desc) && (lean_only || !(clustered && ps.mode == MODE_LANE))) {
                 rc = ps.var >= 3 && ps.var <= 6 ? setup_lean_real(r, dbl, tabs) : setup_lean(r, ps, dbl, blue_n, tabs, order);
                 if (rc) return fail(rc);
                 if (ps.real && r.lean) {
@@ -2054,7 +2057,6 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
                 }
                 if (r.lean && ps.note != "bluestein-B1") ++order;   // (B1 and A2 are one launch)
             }
-            bool ok = line_info(dbl, ps.L, ps.mode, ps.var, &li);
             if (!ok && !r.lean) {
                 set_error("no kernel instantiation for pass " + ps.note + " L=" + std::to_string(ps.L));
                 return fail(RK_ERR_UNSUPPORTED);
