@@ -329,7 +329,9 @@ RK_API int rk_fft1d_c64_noalloc(void* out, const void* in, int64_t n, int64_t ba
  * a batch replaces N such calls.  Every pass of every member must be a line pass with
  * a compiled batched variant (complex64; power-of-two lengths up to 8192 along the
  * contiguous axis, 16 to 256 along strided axes; no plane
- * passes: plan the members with RK_FLAG_NO_PLANE), else RK_ERR_UNSUPPORTED.  A plan
+ * passes: plan the members with RK_FLAG_NO_PLANE), else RK_ERR_UNSUPPORTED.  For a member
+ * made without RK_FLAG_BATCHABLE whose passes only the lean kernels do (mixed radix, long
+ * Bluestein axes) the batch makes and keeps a plan of general passes.  A plan
  * may appear once per batch.  The batch keeps pointers to the plans: destroy it
  * before them.  Calls of one batch must be stream-ordered (one stream, or ordered by
  * the caller); each call waits for the host staging slot it reuses (4 in flight).

@@ -20,6 +20,7 @@
 #include "rk_async.cuh"
 #include "rk_internal.h"
 #include "rk_kernels.cuh"
+#include "rk_lean.h"
 
 namespace rk {
 
@@ -190,6 +191,7 @@ int build_call_params(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs
 struct rk_batch {
     static constexpr int RING = 4;
     std::vector<rk_fft_plan*> plans;
+    std::vector<rk_fft_plan*> own;             // general forms that stand in for members
     std::vector<int> first;                    // first batch pass of each member
     std::vector<rk::BatchPass> passes;         // host copy, pointers patched per call
     std::vector<rk::BatchTask> tasks;
@@ -228,6 +230,20 @@ extern "C" int rk_batch_create(rk_fft_plan* const* plans, int32_t nplans, rk_bat
         for (int j = 0; j < i; ++j)
             if (plans[j] == p)
                 return fail(RK_ERR_INVALID, "rk_batch_create: a plan appears twice (its temporaries would be shared)");
+        // Mixed-radix and three-pass Bluestein passes have lean bodies only, and the tile bodies
+        // here would run their parameters as plain FFTs: the plan's general form, made with
+        // RK_FLAG_NO_TMA, stands in for it.
+        bool only = false;
+        for (const PassRec& r : p->passes) only = only || (r.lean && r.lean->only && !r.dbl);
+        if (only) {
+            rk_fft_desc d = p->desc;
+            d.flags |= RK_FLAG_NO_TMA;
+            rk_fft_plan* general = nullptr;
+            const int rc = rk_fft_plan_create(&d, &general);
+            if (rc) return fail(rc, std::string("rk_batch_create: ") + rk_last_error());
+            b->own.push_back(general);
+            p = general;
+        }
         b->plans.push_back(p);
         maxlevel = std::max<int>(maxlevel, (int)p->passes.size());
         for (const PassRec& r : p->passes) {
@@ -242,7 +258,7 @@ extern "C" int rk_batch_create(rk_fft_plan* const* plans, int32_t nplans, rk_bat
     b->first.resize(nplans);
     for (int i = 0; i < nplans; ++i) {
         b->first[i] = (int)b->passes.size();
-        const rk_fft_plan* p = plans[i];
+        const rk_fft_plan* p = b->plans[i];
         for (size_t k = 0; k < p->passes.size(); ++k) {
             const PassRec& r = p->passes[k];
             BatchPass bp;
@@ -258,7 +274,7 @@ extern "C" int rk_batch_create(rk_fft_plan* const* plans, int32_t nplans, rk_bat
     }
     for (int lvl = 0; lvl < maxlevel; ++lvl)
         for (int i = 0; i < nplans; ++i)
-            if (lvl < (int)plans[i]->passes.size()) {
+            if (lvl < (int)b->plans[i]->passes.size()) {
                 const int bpi = b->first[i] + lvl;
                 for (int64_t blk = 0; blk < b->passes[bpi].nblocks; ++blk) b->tasks.push_back(BatchTask{bpi, 0, blk});
             }
@@ -363,6 +379,7 @@ extern "C" int rk_batch_destroy(rk_batch* b) {
     cudaFree(b->d_tasks);
     cudaFree(b->d_counters);
     if (b->h_pinned) cudaFreeHost(b->h_pinned);
+    for (rk_fft_plan* p : b->own) rk_fft_plan_destroy(p);
     delete b;
     return RK_OK;
 }

@@ -114,6 +114,7 @@ struct LeanPass {
     std::shared_ptr<const LeanPass> second;
     void* mid = nullptr;
     bool fuse_next = false;   // does the next pass' work as well (rows of the three-pass form)
+    bool only = false;        // the pass' general parameters do not describe its whole work
 };
 
 // Mixed-radix passes: the kernel of a mode; real (contiguous lines): 1 RFFT, 2 IRFFT

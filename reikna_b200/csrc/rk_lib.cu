@@ -1004,6 +1004,7 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
         if (!lean_blue_info(dbl, r.L, r.mode, bvar, &lp->info)) return RK_OK;
         lp->blue = true;
         lp->fuse_next = bvar == 3;
+        lp->only = bvar > 1;
         q.blue_n = (uint32_t)blue_n;
         q.jB = (uint32_t)(bvar == 4 ? p.ld.jB : bvar == 5 ? p.st.jB : 1);
         q.chirp = bvar == 5 ? p.st.chirp : p.ld.chirp;
@@ -1271,6 +1272,7 @@ template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int or
     q.mix_nl = x.nl;
     q.nlines = (uint32_t)p.nlines;
     q.rev = order & 1;
+    lp->only = true;
     r.lean = lp;
     return RK_OK;
 }

@@ -9,7 +9,7 @@ import math
 import numpy
 import pytest
 
-from helpers import fft_bound
+from helpers import fft_bound, normal_array, rel_l2
 
 gpu = pytest.mark.gpu
 
@@ -43,3 +43,38 @@ def test_bluestein_axis_after_a_clustered_plane(cuda, shape, dtype, notes):
         call(None, out, x, inverse)
         ref = (torch.fft.ifftn if inverse else torch.fft.fftn)(x.to(torch.complex128))
         assert _rel(out, ref) < fft_bound(dtype, math.prod(shape))
+
+
+@gpu
+@pytest.mark.parametrize("shape,axis", [((3, 16001), 1), ((5, 1000), 1), ((100, 6), 0), ((7, 3001), 1)])
+def test_batch_of_plans_without_the_batchable_flag(rng, cuda, shape, axis):
+    """Members whose own passes are lean-only (three-pass Bluestein, mixed radix) and one
+    whose pass has a tile body, beside a plain member."""
+    import torch
+
+    from reikna_b200 import _native as N
+
+    sizes = [(shape, axis), ((16, 512), 1)]
+    xs = [normal_array(rng, s, numpy.complex64) for s, _ in sizes]
+    ts = [torch.from_numpy(x).to(cuda) for x in xs]
+    outs = [torch.empty_like(t) for t in ts]
+    batch = N.Batch([N.Plan(N.desc(N.FMT_C64, s, (a,))) for s, a in sizes])
+    for inverse in (0, 1):
+        batch.execute([([o.data_ptr()], [t.data_ptr()], inverse, ()) for o, t in zip(outs, ts)],
+                      stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        for x, o, (s, a) in zip(xs, outs, sizes):
+            ref = (numpy.fft.ifft if inverse else numpy.fft.fft)(x.astype(numpy.complex128), axis=a)
+            assert rel_l2(o.cpu().numpy(), ref) < fft_bound(numpy.complex64, s[a])
+    assert N.device_status(clear=True) == 0
+    batch.close()
+
+
+@gpu
+def test_batch_refuses_one_pass_real_members(cuda):
+    from reikna_b200 import _native as N
+
+    d = N.desc(N.FMT_C64, (5, 97), (1,), N.FLAG_REAL_POST | N.FLAG_REAL_ANY)
+    d.input, d.output = N.edge(N.FMT_C64, (5, 97)), N.edge(N.FMT_C64, (5, 98))
+    with pytest.raises(NotImplementedError):
+        N.Batch([N.Plan(d)])
