@@ -206,7 +206,10 @@ RK_API int rk_fft_plan_destroy(rk_fft_plan* plan);
  *   CTA}; *smem = dynamic shared memory bytes of a CTA.
  * rk_fft_plan_set_pass_kernel: load a cubin `image` (size bytes) holding the
  *   extern "C" kernel `name` with the pass's launch shape and a single
- *   `rk::PassParams` argument, and run pass `index` with it from now on.
+ *   `rk::PassParams` argument, and run pass `index` with it from now on.  Passes with a
+ *   kernel of another launch shape (plane, TMA-fed, tensor-core, pair) or none of the
+ *   general ones (mixed radix, long Bluestein axes, one-pass real transforms of any
+ *   length) take none: RK_ERR_UNSUPPORTED.
  * rk_fft_execute_user: rk_fft_execute plus up to 8 64-bit words per edge handed to
  *   the user code (array pointers and scalar bit patterns, as the host that generated
  *   the code laid them out).

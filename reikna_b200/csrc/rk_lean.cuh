@@ -530,6 +530,8 @@ template <typename T, int L, int MODE, int VAR, bool TW4> struct LeanLauncher {
         r.segments = &lean_segments<C, L>;
         r.tw_elems = LeanTw<L, typename C::P>::total();
         r.nl = C::NL;
+        r.nt = C::NT;
+        r.smem = C::SMEM;
         return r;
     }
 };

@@ -101,7 +101,9 @@ struct LeanInfo {
     cudaError_t (*prepare)();
     void (*segments)(std::vector<StageSeg>&);
     int tw_elems;
-    int nl;
+    int nl;                // lines, threads and dynamic shared memory of a CTA
+    int nt;
+    size_t smem;
 };
 // What a plan keeps for a pass that a lean kernel takes
 struct LeanPass {

@@ -306,6 +306,8 @@ template <typename T, int L, int MODE, int VAR> struct LeanBlueLauncher {
         r.segments = &lean_segments<C, L>;
         r.tw_elems = LeanTw<L, typename C::P>::total();
         r.nl = C::NL;
+        r.nt = C::NT;
+        r.smem = C::SMEM;
         return r;
     }
 };

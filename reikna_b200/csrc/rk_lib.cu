@@ -2394,6 +2394,12 @@ int rk_fft_plan_pass_info(const rk_fft_plan* plan, int32_t index, int32_t* info,
     info[6] = r.user_bits;
     info[7] = r.kind == PK_LINE ? r.li.nl : 0;
     *smem = (int64_t)(r.kind == PK_LINE ? r.li.smem : r.pi.smem);
+    if (r.lean && !r.li.fn && r.kind == PK_LINE) {   // (no general kernel of this length)
+        const LeanPass& lp = *r.lean;
+        info[5] = lp.prm.mix ? (int32_t)lp.prm.mix_nt : lp.info.nt;
+        info[7] = lp.prm.mix ? (int32_t)lp.prm.mix_nl : lp.info.nl;
+        *smem = lp.prm.mix ? lp.prm.mix_smem : lp.info.smem;
+    }
     return RK_OK;
 }
 
@@ -2403,7 +2409,14 @@ int rk_fft_plan_set_pass_kernel(rk_fft_plan* plan, int32_t index, const void* im
         return RK_ERR_INVALID;
     }
     PassRec& r = plan->passes[index];
-    if (r.kind != PK_LINE || r.use_tc || r.use_tma || r.pair_first) {
+    bool plain = r.kind == PK_LINE && !r.use_tc && !r.use_tma && !r.pair_first && r.li.fn;
+    if (plain && r.lean) {
+        // the general kernel in its place has to be one that takes an installed kernel too
+        PassRec general = r;
+        setup_tma(general, r.dbl, 1);
+        plain = !r.lean->only && !(general.use_tma && r.var == 0);
+    }
+    if (!plain) {
         set_error("rk_fft_plan_set_pass_kernel: only plain line passes take an installed kernel");
         return RK_ERR_UNSUPPORTED;
     }
@@ -2425,6 +2438,8 @@ int rk_fft_plan_set_pass_kernel(rk_fft_plan* plan, int32_t index, const void* im
     if (r.user_lib) cudaLibraryUnload((cudaLibrary_t)r.user_lib);
     r.user_lib = lib;
     r.user_kern = (const void*)kern;
+    r.lean.reset();
+    for (auto& chain : plan->chain) chain.reset();   // rk_fft_call runs the installed kernel, too
     return RK_OK;
 }
 

@@ -78,3 +78,52 @@ def test_batch_refuses_one_pass_real_members(cuda):
     d.input, d.output = N.edge(N.FMT_C64, (5, 97)), N.edge(N.FMT_C64, (5, 98))
     with pytest.raises(NotImplementedError):
         N.Batch([N.Plan(d)])
+
+
+MARK = """#include "rk_params.h"
+extern "C" __global__ void mark(const rk::PassParams p) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ((float2*)p.st.ptr)[0] = make_float2(42.0f, 0.0f);
+}
+"""
+
+
+@gpu
+def test_an_installed_kernel_runs_in_every_call(cuda):
+    """rk_fft_call and rk_fft_execute both leave the prepared lean launches for it."""
+    import torch
+
+    from reikna_b200 import _native as N
+    from reikna_b200 import _rtc
+
+    plan = N.Plan(N.desc(N.FMT_C64, (3, 64, 5), (1,)))
+    x = torch.ones((3, 64, 5), dtype=torch.complex64, device=cuda)
+    stream = torch.cuda.current_stream().cuda_stream
+    out = torch.zeros_like(x)
+    plan.call(out.data_ptr(), x.data_ptr(), 0, stream)
+    torch.cuda.synchronize()
+    assert out[0, 0, 0] == 64
+    plan.set_pass_kernel(0, _rtc.compile_cubin(MARK), "mark")
+    for run in (lambda: plan.call(out.data_ptr(), x.data_ptr(), 0, stream),
+                lambda: plan.execute([out.data_ptr()], [x.data_ptr()], stream=stream)):
+        out.zero_()
+        run()
+        torch.cuda.synchronize()
+        assert out[0, 0, 0] == 42 and torch.count_nonzero(out) == 1
+
+
+@gpu
+@pytest.mark.parametrize("shape,axis,passes", [((5, 1000), 1, 1), ((3, 16001), 1, 4), ((64, 1024), 1, 1), ((4, 1024, 64), 1, 1),
+                                               ((3, 300, 5), 1, 1)])
+def test_passes_without_a_general_kernel_take_no_installed_one(cuda, shape, axis, passes):
+    """Mixed-radix and three-pass Bluestein passes, and lines the TMA-fed kernel would run;
+    their launch shapes are those of the kernels that do run."""
+    from reikna_b200 import _native as N
+    from reikna_b200 import _rtc
+
+    plan = N.Plan(N.desc(N.FMT_C64, shape, (axis,)))
+    info = plan.pass_info()
+    assert len(info) == passes and all(p["nt"] > 0 and p["nl"] > 0 for p in info)
+    cubin = _rtc.compile_cubin(MARK)
+    for i in range(passes):
+        with pytest.raises(NotImplementedError, match="plain line passes"):
+            plan.set_pass_kernel(i, cubin, "mark")
