@@ -181,7 +181,10 @@ RK_API int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** plan);
  * inverse: 0 forward (exp(-i...)), 1 inverse normalised by 1/N (IFFT(FFT(x)) = x).
  * scalars: n_scalars complex values, as (re, im) pairs of doubles, for the runtime
  * scalar slots referenced by the edges.
- * Output may alias input. */
+ * The output may be the input array.  Arrays that overlap in another way are for real
+ * transforms of the last axis (RK_FLAG_REAL_POST / _PRE, real inputs on the half-length
+ * route) only: those then read a private copy of the input, in memory the plan keeps from
+ * the first such call on. */
 RK_API int rk_fft_execute(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs,
                    const void* const* inputs, int32_t n_inputs, int32_t inverse,
                    const double* scalars, int32_t n_scalars, void* stream);

@@ -150,9 +150,11 @@ struct rk_fft_plan {
     int64_t device_bytes = 0;
     double n_total = 1.0;          // inverse normalisation
     bool alias_hazard = false;     // single remapping pass: in == out needs a copy
+    bool alias_any = false;        // so does every other overlap of input and output
     void* alias_tmp = nullptr;
     int64_t in_extent_bytes = 0;   // bytes spanned by the input array (alias copy)
     int64_t in2_extent_bytes = 0;
+    int64_t out_extent_bytes = 0;
     // per-pass event profiling (rk_fft_profile)
     std::vector<cudaEvent_t> prof_ev;   // 2 * passes * max_calls
     int32_t prof_max = 0, prof_used = 0;

@@ -1559,6 +1559,24 @@ int build_call_params(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs
                       std::vector<PassParams>& out, std::vector<char>* tma_ok, const uint64_t* user_in,
                       int32_t n_user_in, const uint64_t* user_out, int32_t n_user_out);
 
+// Whether a single pass stages every overlap of its arrays, not only equal pointers: the
+// real transforms, whose two arrays have lines of different lengths, and lean passes in
+// place of several general ones, which went through temporaries.
+static bool overlap_staged(const PassRec& r) {
+    if (r.kind != PK_LINE) return false;
+    if ((r.var >= 3 && r.var <= 6) || (r.lean && r.lean->prm.rmix)) return true;
+    if (!r.lean || (r.li.fn && !r.lean->only)) return false;
+    const int64_t M = 2 * bpow2(r.lean->prm.mix ? r.L : r.lean->prm.blue_n);
+    return M > (r.mode == MODE_POS ? pos_max(r.dbl) : r.dbl ? lane_max(r.dbl) : 2048);
+}
+
+// Whether the call's input is read from a private copy.
+static bool needs_staging(const rk_fft_plan* plan, const void* in, const void* out) {
+    if (in == out) return plan->alias_hazard;
+    return plan->alias_any && (const char*)in < (const char*)out + plan->out_extent_bytes &&
+           (const char*)out < (const char*)in + plan->in_extent_bytes;
+}
+
 // The launches of one direction of a plan whose passes are all lean and whose edges take
 // one array each and no scalars: what rk_fft_call does per call is then to fill in the
 // pointers (building each pass' general parameters, 1.7 KB a pass, and the conversion
@@ -1572,7 +1590,8 @@ static std::shared_ptr<const LeanChain> build_chain(rk_fft_plan* plan, int inver
     for (const PassRec& r : plan->passes)
         if (!r.lean || r.pair_first || r.user_kern) return nullptr;
     // stand-ins for the user's pointers, aligned and apart
-    char *in = (char*)0x10000000, *out = (char*)0x20000000;
+    const int64_t apart = 0x10000000;
+    char *in = (char*)apart, *out = in + (plan->in_extent_bytes / apart + 1) * apart;
     void* outs[1] = {out};
     const void* ins[1] = {in};
     std::vector<PassParams> prm;
@@ -2106,7 +2125,9 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
             same = a.strides[i] == b.strides[i] && a.shift[i] == b.shift[i] && a.shape[i] == b.shape[i] &&
                    (!fmt_is_pair(a.format) || a.strides2[i] == b.strides2[i]);
         plan->alias_hazard = !same || !plan->passes[0].inplace_safe;
+        plan->alias_any = overlap_staged(plan->passes[0]);
         plan->in_extent_bytes = edge_extent_bytes(desc->input, 0);
+        plan->out_extent_bytes = edge_extent_bytes(desc->output, 0);
         if (fmt_is_pair(desc->input.format)) plan->in2_extent_bytes = edge_extent_bytes(desc->input, 1);
     }
     // set launch attributes now (cudaFuncSetAttribute is not allowed during capture)
@@ -2249,11 +2270,16 @@ int build_call_params(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs
     void* out1 = need_out > 1 ? outputs[1] : nullptr;
 
     // in-place call of a single remapping pass: read from a private copy
-    if (plan->alias_hazard && in0 && out0 &&
-        (in0 == out0 || (in1 && (in1 == out0 || (out1 && in1 == out1))) || (out1 && in0 == out1))) {
+    if (in0 && out0 &&
+        (needs_staging(plan, in0, out0) ||
+         (plan->alias_hazard && ((in1 && (in1 == out0 || (out1 && in1 == out1))) || (out1 && in0 == out1))))) {
         const int64_t need = plan->in_extent_bytes + plan->in2_extent_bytes + 256;
         if (!plan->alias_tmp) {
+            // (the first such call may be one that a stream captures)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            CK(cudaThreadExchangeStreamCaptureMode(&mode));
             cudaError_t e = cudaMalloc(&plan->alias_tmp, (size_t)need);
+            cudaThreadExchangeStreamCaptureMode(&mode);
             if (e != cudaSuccess) {
                 set_error("in-place staging allocation failed");
                 return RK_ERR_NOMEM;
@@ -2451,7 +2477,7 @@ int rk_fft_execute(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs, c
 
 int rk_fft_call(rk_fft_plan* plan, void* output, const void* input, int32_t inverse, void* stream) {
     const LeanChain* chain = plan ? plan->chain[inverse ? 1 : 0].get() : nullptr;
-    if (!chain || !output || !input || plan->prof_used < plan->prof_max || (plan->alias_hazard && input == output))
+    if (!chain || !output || !input || plan->prof_used < plan->prof_max || needs_staging(plan, input, output))
         return rk_fft_execute(plan, &output, 1, &input, 1, inverse, nullptr, 0, stream);
     for (const LeanChain::Item& it : chain->items) {
         LeanParams q = it.prm;

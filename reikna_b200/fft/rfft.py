@@ -7,7 +7,8 @@ N/2 without the last bin), like ``numpy.fft.rfft`` along the last axis.
 ``IRFFT(arr_t)``: complex (..., H + 1) -> real (..., 2H), like ``numpy.fft.irfft``.
 ``APRFFT(arr_t)``: real (..., N/2), the first half of a signal with
 x[n + N/2] = -x[n] -> its N/4 odd harmonics.  ``IAPRFFT(arr_t)``: the inverse.
-Signatures ``(output:o, input:i)``.
+Signatures ``(output:o, input:i)``.  The two arrays may overlap in any way: ``RFFT`` and
+``IRFFT`` then transform a private copy of the input.
 
 As in the reference, the real array is read by a complex FFT of half its length as
 interleaved (re, im) pairs.  When that half length is a power of two (8 to 8192

@@ -127,3 +127,81 @@ def test_passes_without_a_general_kernel_take_no_installed_one(cuda, shape, axis
     for i in range(passes):
         with pytest.raises(NotImplementedError, match="plain line passes"):
             plan.set_pass_kernel(i, cubin, "mark")
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.float32, numpy.float64])
+@pytest.mark.parametrize("n", [200, 194, 256, 3000])
+@pytest.mark.parametrize("start", [0, 8, 600, 6000])
+def test_real_transforms_of_overlapping_arrays(rng, cuda, dtype, n, start):
+    """RFFT and IRFFT (mixed-radix, Bluestein and power-of-two bodies) whose arrays share
+    memory, the second one `start` samples behind the first or in front of it."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import IRFFT, RFFT
+
+    rows = 2**18 // n
+    cdt = torch.complex64 if dtype == numpy.float32 else torch.complex128
+    bound = fft_bound(numpy.complex64 if dtype == numpy.float32 else numpy.complex128, n)
+    x = rng.standard_normal((rows, n)).astype(dtype)
+    spec = numpy.fft.rfft(x.astype(numpy.float64), axis=1)
+    bins = rows * (n // 2 + 1)
+    forward = RFFT(ArrayMetadata((rows, n), dtype)).compile()
+    inverse = IRFFT(ArrayMetadata((rows, n // 2 + 1), spec.astype(numpy.complex64).dtype if dtype == numpy.float32 else spec.dtype)).compile()
+    for behind in (False, True):
+        buf = torch.zeros(rows * n + 2 * rows + start, dtype=torch.float32 if dtype == numpy.float32 else torch.float64, device=cuda)
+        a, b = (0, start) if behind else (start, 0)
+        real = buf[a:a + rows * n].view(rows, n)
+        half = buf[b:b + 2 * bins].view(cdt).view(rows, n // 2 + 1)
+        real.copy_(torch.from_numpy(x))
+        forward(None, half, real)
+        torch.cuda.synchronize()
+        assert rel_l2(half.cpu().numpy(), spec) < bound
+        half.copy_(torch.from_numpy(spec).to(cdt))
+        inverse(None, real, half)
+        torch.cuda.synchronize()
+        assert rel_l2(real.cpu().numpy(), x) < bound
+
+
+@gpu
+@pytest.mark.parametrize("dtype,n,cols", [(numpy.complex64, 1500, 40), (numpy.complex128, 257, 40), (numpy.complex128, 1500, 24)])
+def test_long_strided_lines_shifted_within_their_array(rng, cuda, dtype, n, cols):
+    """Lean passes in place of several general ones, which went through temporaries."""
+    import torch
+
+    from reikna_b200.fft import FFT
+
+    x = normal_array(rng, (n, cols), dtype)
+    ref = numpy.fft.fft(x.astype(numpy.complex128), axis=0)
+    for a, b in ((0, 1), (1, 0)):
+        buf = torch.zeros((n + 1, cols), dtype=torch.complex64 if dtype == numpy.complex64 else torch.complex128, device=cuda)
+        src, dst = buf[a:a + n], buf[b:b + n]
+        src.copy_(torch.from_numpy(x))
+        FFT(src, axes=(0,)).compile()(None, dst, src)
+        torch.cuda.synchronize()
+        assert rel_l2(dst.cpu().numpy(), ref) < fft_bound(dtype, n)
+
+
+@gpu
+def test_first_overlapping_call_inside_a_capture(rng, cuda):
+    """The private copy is allocated by the call that needs it first, also where a stream
+    captures that call."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import RFFT
+
+    rows, n = 300, 200
+    x = rng.standard_normal((rows, n)).astype(numpy.float32)
+    buf = torch.zeros(rows * (n + 2), dtype=torch.float32, device=cuda)
+    real, half = buf[:rows * n].view(rows, n), buf.view(torch.complex64).view(rows, n // 2 + 1)
+    call = RFFT(ArrayMetadata((rows, n), numpy.float32)).compile()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(None, half, real)
+    for _ in range(2):
+        real.copy_(torch.from_numpy(x))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert rel_l2(half.cpu().numpy(), numpy.fft.rfft(x.astype(numpy.float64), axis=1)) < fft_bound(numpy.complex64, n)
