@@ -84,7 +84,9 @@ extern "C" {
                                 accumulate) for 256- and 1024-point contiguous complex64
                                 line passes; others run as usual */
 #define RK_FLAG_PLANE_WIDE 8 /* plane pass on twice as many CTAs per cluster (tuning) */
-#define RK_FLAG_NO_TMA 16    /* never use the persistent TMA-fed line passes */
+#define RK_FLAG_NO_TMA 16    /* general kernels only: no persistent TMA-fed line passes, and none of
+                                the lean ones (plain lines, planes as rows and columns, mixed
+                                radix, three-pass Bluestein, RK_FLAG_REAL_ANY) */
 #define RK_FLAG_PAIR 32      /* two innermost power-of-two axes: row and column passes in one
                                 plane-ordered launch instead of the clustered plane pass */
 #define RK_FLAG_REAL_POST 64 /* forward transform of the last axis (length L = N/2, a power of two
@@ -212,7 +214,8 @@ RK_API int rk_fft_plan_destroy(rk_fft_plan* plan);
  *   `rk::PassParams` argument, and run pass `index` with it from now on.  Passes with a
  *   kernel of another launch shape (plane, TMA-fed, tensor-core, pair) or none of the
  *   general ones (mixed radix, long Bluestein axes, one-pass real transforms of any
- *   length) take none: RK_ERR_UNSUPPORTED.
+ *   length) take none: RK_ERR_UNSUPPORTED.  A plan made with RK_FLAG_NO_TMA has general
+ *   line passes throughout.
  * rk_fft_execute_user: rk_fft_execute plus up to 8 64-bit words per edge handed to
  *   the user code (array pointers and scalar bit patterns, as the host that generated
  *   the code laid them out).

@@ -9,8 +9,9 @@ measured on the caller's own arguments and the fastest is kept:
   (16-CTA clusters, 16 rows a CTA), the same on twice-as-wide clusters
   (``FLAG_PLANE_WIDE``), a row pass and a column pass in one plane-ordered persistent
   launch (``FLAG_PAIR``), or separate line passes (``FLAG_NO_PLANE``);
-* operand staging: persistent TMA-fed line passes or plain per-tile loads
-  (``FLAG_NO_TMA``);
+* the kernels of plain line passes: the lean, mixed-radix and three-pass Bluestein ones,
+  with the persistent TMA-fed passes behind planes, or the general per-tile kernel and
+  Bluestein throughout (``FLAG_NO_TMA``);
 * threads per transform and radix plan of 8192-point Bluestein lines: one CTA of 256
   threads with 32 elements a thread (the default), 16 on 512 (``FLAG_R16``), or a
   two-CTA cluster a line, each CTA one half of the padded spectrum
@@ -32,7 +33,8 @@ import hashlib
 from . import _native as N
 from .batch import _load_cache, _store_cache
 
-_VERSION = b"fft-tune-1"
+# bumped when the kernels behind the candidates change, so that older choices are re-tuned
+_VERSION = b"fft-tune-2"
 
 
 def candidates(comp, allow_split: bool = False) -> list[int]:

@@ -37,8 +37,9 @@ from . import _native as N
 
 MODES = ("calls", "graph", "graph_par", "persistent")
 
-# bumped when the candidate set changes, so that older cached choices are re-tuned
-_TUNE_VERSION = b"3"
+# bumped when the candidate set or the kernels behind it change, so that older cached choices
+# are re-tuned
+_TUNE_VERSION = b"4"
 
 
 def _cache_path() -> Path:

@@ -205,3 +205,20 @@ def test_first_overlapping_call_inside_a_capture(rng, cuda):
         graph.replay()
         torch.cuda.synchronize()
         assert rel_l2(half.cpu().numpy(), numpy.fft.rfft(x.astype(numpy.float64), axis=1)) < fft_bound(numpy.complex64, n)
+
+
+def test_choices_tuned_on_earlier_kernels_are_tuned_again():
+    import hashlib
+
+    from reikna_b200 import _native as N
+    from reikna_b200 import autotune, batch
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import FFT
+
+    comp = FFT(ArrayMetadata((1000, 1000), numpy.complex64))
+    desc = bytes(comp.native_descriptor(0)[0])
+    assert autotune._key(comp, False) != hashlib.sha256(b"fft-tune-1" + desc).hexdigest()[:32]
+    assert batch._desc_key([comp.native_descriptor(0)[0]]) != hashlib.sha256(b"3" + desc).hexdigest()[:32]
+    # the flag those choices held for most plans turns the kernels of today off
+    assert [p["note"] for p in comp.describe(0)["passes"]] == ["mixed", "mixed"]
+    assert "mixed" not in [p["note"] for p in comp.describe(N.FLAG_NO_TMA)["passes"]]
