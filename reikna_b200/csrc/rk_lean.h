@@ -45,6 +45,7 @@ struct MixPlan {
     uint32_t inplace;      // a thread has at most one butterfly a stage
     uint32_t bufs;         // buffers: one in place, or with nothing between first and last stage
     FastDiv r0;
+    FastDiv prdiv;         // by n / 2 + 1: bin pairs of a line (real transforms)
     MixStage stage[MIX_STAGES];
 };
 

@@ -257,6 +257,23 @@ __device__ __forceinline__ void mix_radix(const LeanParams& p, const MixPlan& x,
 #undef RK_MIX
 }
 
+// f(line, k) for the bin pairs k, n - k (k <= n / 2) of the tile's lines, one after another
+// over the CTA's threads.  Line by line, 26 of 384 threads had work at 50 samples: 41943 lines
+// of them, float32, RFFT 23.6 -> 6.6 us and IRFFT 26.5 -> 6.9, 116508 lines of 18 samples
+// 52.3 -> 7.1 and 63.5 -> 7.1.  (A tile of one line needs no division: with one, IRFFTs of 3000
+// to 12000 float64 samples took 3% longer.)
+template <class F> __device__ __forceinline__ void mix_pairs(const MixPlan& x, uint32_t lines, F f) {
+    const uint32_t pairs = x.prdiv.d;
+    if (x.nl == 1) {
+        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) f(0u, k);
+    } else {
+        for (uint32_t i = threadIdx.x; i < lines * pairs; i += blockDim.x) {
+            const uint32_t ln = fd_div(x.prdiv, i);
+            f(ln, i - ln * pairs);
+        }
+    }
+}
+
 // The real-spectrum step of the tile's lines: z (pitch and pads of the tile) to bins
 // X[0 .. n) and, where stored, X[n].  w_k = exp(-i pi k / n) in rmix.
 template <typename T>
@@ -264,20 +281,18 @@ __device__ __forceinline__ void mix_bins_out(const LeanParams& p, const MixPlan&
                                              uint32_t valid) {
     using V = cplx<T>;
     const V* wk = reinterpret_cast<const V*>(p.rmix);
-    const uint32_t n = x.n, pairs = n / 2 + 1;
+    const uint32_t n = x.n;
     auto at = [&](uint32_t k) { return k + (x.pad ? fd_div(x.r0, k) : 0u); };
-    for (uint32_t ln = 0; ln < valid; ++ln) {
+    mix_pairs(x, valid, [&](uint32_t ln, uint32_t k) {
         const V* zl = z + ln * x.pitch;
         V* out = reinterpret_cast<V*>(p.st.base + off_st[ln]);
-        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) {
-            V o[2];
-            real_pair<T>(zl[at(k)], zl[at(k == 0 ? 0 : n - k)], __ldg(wk + k), T(0.5), o[0], o[1]);
-            if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
-            if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
-            out[k] = o[0];
-            if (k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * k < n) out[n - k] = o[1];
-        }
-    }
+        V o[2];
+        real_pair<T>(zl[at(k)], zl[at(k == 0 ? 0 : n - k)], __ldg(wk + k), T(0.5), o[0], o[1]);
+        if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
+        if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
+        out[k] = o[0];
+        if (k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * k < n) out[n - k] = o[1];
+    });
 }
 
 // The inverse step: bins of the tile's lines to the half-length spectrum, lines of n points.
@@ -285,24 +300,22 @@ template <typename T>
 __device__ __forceinline__ void mix_bins_in(const LeanParams& p, const MixPlan& x, cplx<T>* z, const uint32_t* off_ld) {
     using V = cplx<T>;
     const V* wk = reinterpret_cast<const V*>(p.rmix);
-    const uint32_t n = x.n, pairs = n / 2 + 1;
-    for (uint32_t ln = 0; ln < x.nl; ++ln) {
+    const uint32_t n = x.n;
+    mix_pairs(x, x.nl, [&](uint32_t ln, uint32_t k) {
         const V* in = reinterpret_cast<const V*>(p.ld.base + off_ld[ln]);
         V* zl = z + ln * n;
-        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) {
-            V y[2] = {in[k], in[n - k]}, a, b;
-            if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, y);
-            if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(y);
-            if (k == 0) {
-                // bins 0 and n of a real signal are real
-                y[0].y = T(0);
-                y[1].y = T(0);
-            }
-            real_pair<T>(y[0], y[1], __ldg(wk + k), T(0.5), a, b);
-            zl[k] = a;
-            if (k > 0 && 2 * k < n) zl[n - k] = b;
+        V y[2] = {in[k], in[n - k]}, a, b;
+        if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, y);
+        if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(y);
+        if (k == 0) {
+            // bins 0 and n of a real signal are real
+            y[0].y = T(0);
+            y[1].y = T(0);
         }
-    }
+        real_pair<T>(y[0], y[1], __ldg(wk + k), T(0.5), a, b);
+        zl[k] = a;
+        if (k > 0 && 2 * k < n) zl[n - k] = b;
+    });
 }
 
 // REAL 1: the real-spectrum step after the FFT (RFFT: sample pairs in, bins out); 2: the

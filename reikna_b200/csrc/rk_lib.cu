@@ -1150,6 +1150,7 @@ static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int
     x.ns = ns;
     x.pad = mode == MODE_POS && r[0] % 2 == 0;
     x.r0 = fast_div((uint32_t)r[0]);
+    x.prdiv = fast_div((uint32_t)(n / 2 + 1));
     x.pitch = (uint32_t)(n + (x.pad ? n / r[0] : 0));
     uint32_t P = 1, tw = 0;
     for (int s = 0; s < ns; ++s) {

@@ -424,3 +424,32 @@ def test_dependent_launches_in_graphs_and_streams(rng, cuda):
         ref = 2 * numpy.fft.fftn(src.cpu().numpy().astype(numpy.complex128))
         assert rel_l2(c.cpu().numpy(), ref) < fft_bound(numpy.complex64, src.numel())
         assert rel_l2(a.cpu().numpy(), src.cpu().numpy()) < 2 * fft_bound(numpy.complex64, 96 * 250)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.float32, numpy.float64])
+@pytest.mark.parametrize("half", [9, 13, 25, 30, 50, 100])
+@pytest.mark.parametrize("rows", [81, 4099])
+def test_many_short_real_lines(rng, cuda, dtype, half, rows):
+    """Tiles of many lines, whose bin pairs are spread over the CTA's threads; whole tiles
+    and a partial last one, with and without the Nyquist bin."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import IRFFT, RFFT
+
+    x = rng.standard_normal((rows, 2 * half)).astype(dtype)
+    t = torch.from_numpy(x).to(cuda)
+    cdt = torch.complex64 if dtype == numpy.float32 else torch.complex128
+    bound = fft_bound(numpy.complex64 if dtype == numpy.float32 else numpy.complex128, 2 * half)
+    ref = numpy.fft.rfft(x.astype(numpy.float64), axis=1)
+    for last in (False, True):
+        out = torch.full((rows, half + (0 if last else 1)), float("nan"), dtype=cdt, device=cuda)
+        RFFT(ArrayMetadata((rows, 2 * half), dtype), dont_store_last=last).compile()(None, out, t)
+        torch.cuda.synchronize()
+        assert rel_l2(out.cpu().numpy(), ref[:, :out.shape[1]]) < bound
+    spec = torch.from_numpy(ref).to(cdt).to(cuda)
+    back = torch.full((rows, 2 * half), float("nan"), dtype=t.dtype, device=cuda)
+    IRFFT(spec).compile()(None, back, spec)
+    torch.cuda.synchronize()
+    assert rel_l2(back.cpu().numpy(), x) < 2 * bound
