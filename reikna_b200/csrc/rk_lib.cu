@@ -1295,18 +1295,36 @@ static void plane_split(const rk_fft_desc& d, const PassSpec& p, int mid, PassSp
 // Whether a plane pass runs as two lean line passes, rows then columns, and through which
 // buffer (the pass' own temporary, or the output where the columns can be transformed in
 // place there); -1: the clustered kernel.  While L2 holds the array the second pass costs
-// little and both run far closer to the copy rate than the cluster's exchange lets one pass:
-// 16 x 256 x 256 complex64 12.3 -> 9.6 us, 128 x 256 x 256 51.8 -> 45.1, 64 x 128 x 128 10.3 ->
-// 9.4.  Beyond 64 MB the extra round trip through HBM counts: 4096 x 64 x 64 complex64 71.0 us
-// clustered against 81.1, 512 x 128 x 128 complex128 80.0 against 86.2, and 256 x 256 x 256 in
-// steps over three streams 125 us a step against 138 (alone on one stream the line passes
-// win, 135 against 145); 128 x 128 complex64 planes take the line passes at every size
-// (1024 of them: 82.1 against 85.3).
+// little and both run far closer to the copy rate than the cluster's exchange lets one pass;
+// beyond it the extra round trip through HBM counts, the more so where calls on several
+// streams share L2.  us a call in a captured chain of three arrays' calls, clustered against
+// line passes, and in brackets the same calls on three streams:
+//   complex64   16 x 256 x 256   11.3  9.2 [7.8  4.2]     128 x 256 x 256  52.4 42.2 [45.1 40.3]
+//               64 x 128 x 128    9.2  9.0 [6.3  4.1]    1024 x 128 x 128  84.3 78.0 [76.0 77.0]
+//             1280 x 128 x 128  102.4 99.4 [94.4 98.0]     1536 x 128 x 128  123.7 124.5 [113.0 124.2]
+//               64 x 64 x 64      4.8  5.0 [2.2  2.2]      96 x 64 x 64     4.5  6.1 [2.2  2.5]
+//              148 x 64 x 64      4.8  6.5 [2.9  2.8]     149 x 64 x 64     6.9  6.6 [3.0  2.8]
+//             1024 x 64 x 64     22.4 19.4 [16.5 18.4]   1280 x 64 x 64    24.8 23.9 [20.4 23.8]
+//             2048 x 64 x 64     37.0 38.2 [31.7 38.5]
+//   complex128  64 x 128 x 128   15.9 12.7 [12.2 7.4]     256 x 128 x 128  43.8 42.4 [39.1 38.7]
+//              512 x 128 x 128   80.0 against 86.2        2048 x 64 x 64    94.2 78.5 [86.4 76.8]
+// The lines lie where the loss on one side outweighs the gain on the other (a 64 x 64 plane
+// kernel has one CTA a plane: 65 to 148 planes are one wave of them).  256 x 256 x 256 in steps
+// over three streams takes 125 us a step with planes against 138.  With a third axis behind
+// the planes the line passes win further up (2048 x 128 x 128 complex64 over three axes 443
+// against 343 [429 against 354], 128 x 256 x 256 74.0 62.5 [58.4 61.1]).
 static int plane_mid(const rk_fft_desc& d, const PassSpec& p) {
     const int dbl = d.dtype == RK_FMT_C128;
     if (!lean_allowed(d) || (d.flags & RK_FLAG_PLANE_WIDE)) return -1;
-    const int64_t bytes = p.O * p.L1 * p.L2 * (dbl ? 16 : 8);
-    if (bytes > (int64_t(64) << 20) && (p.L1 == (dbl ? 128 : 64) || p.L1 == 256)) return -1;
+    const int64_t bytes = p.O * p.L1 * p.L2 * (dbl ? 16 : 8), MB = int64_t(1) << 20;
+    const bool last = p.st.buf == SB_OUT;
+    if (!dbl && p.L1 == 64) {
+        if (bytes > (last ? 36 : 64) * MB || (last && p.O > 64 && p.O <= 148)) return -1;
+    } else if (!dbl && p.L1 == 128) {
+        if (last && bytes > 160 * MB) return -1;
+    } else if (p.L1 != 64 && bytes > 64 * MB) {
+        return -1;
+    }
     std::vector<int> mids;
     if (p.st.buf != SB_OUT) {
         mids = {p.st.buf};

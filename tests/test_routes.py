@@ -222,3 +222,26 @@ def test_choices_tuned_on_earlier_kernels_are_tuned_again():
     # the flag those choices held for most plans turns the kernels of today off
     assert [p["note"] for p in comp.describe(0)["passes"]] == ["mixed", "mixed"]
     assert "mixed" not in [p["note"] for p in comp.describe(N.FLAG_NO_TMA)["passes"]]
+
+
+@gpu
+@pytest.mark.parametrize("shape,dtype,launches", [
+    ((64, 64, 64), numpy.complex64, 2), ((65, 64, 64), numpy.complex64, 1), ((148, 64, 64), numpy.complex64, 1),
+    ((149, 64, 64), numpy.complex64, 2), ((1152, 64, 64), numpy.complex64, 2), ((1153, 64, 64), numpy.complex64, 1),
+    ((1280, 128, 128), numpy.complex64, 2), ((1281, 128, 128), numpy.complex64, 1), ((100, 64, 64), numpy.complex128, 2)])
+def test_planes_on_both_sides_of_the_split(cuda, shape, dtype, launches):
+    """Planes as one launch or as rows and columns, where the choice changes."""
+    import torch
+
+    from reikna_b200.core import ArrayMetadata
+    from reikna_b200.fft import FFT
+
+    call = FFT(ArrayMetadata(shape, dtype), axes=(1, 2)).compile()
+    assert call.launches == launches
+    torch.manual_seed(5)
+    x = torch.randn(shape, dtype=torch.complex64 if dtype == numpy.complex64 else torch.complex128, device=cuda)
+    out = torch.empty_like(x)
+    for inverse in (0, 1):
+        call(None, out, x, inverse)
+        ref = (torch.fft.ifftn if inverse else torch.fft.fftn)(x.to(torch.complex128), dim=(1, 2))
+        assert _rel(out, ref) < fft_bound(dtype, shape[1] * shape[2])
