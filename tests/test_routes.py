@@ -245,3 +245,48 @@ def test_planes_on_both_sides_of_the_split(cuda, shape, dtype, launches):
         call(None, out, x, inverse)
         ref = (torch.fft.ifftn if inverse else torch.fft.fftn)(x.to(torch.complex128), dim=(1, 2))
         assert _rel(out, ref) < fft_bound(dtype, shape[1] * shape[2])
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [numpy.complex64, numpy.complex128])
+@pytest.mark.parametrize("shape,axes", [((6, 128, 128), (0, 1, 2)), ((16, 128, 128), (0, 1, 2)), ((5, 64, 64), (0, 1, 2)),
+                                        ((2, 17, 64, 64), (1, 2, 3)), ((5, 256, 256), (0, 1, 2))])
+@pytest.mark.parametrize("shift", [False, True])
+@pytest.mark.parametrize("views", [False, True])
+def test_planes_split_through_a_temporary(rng, cuda, dtype, shape, axes, shift, views):
+    """Planes with another axis behind them: rows and columns through the plan's temporary,
+    then power-of-two, mixed-radix or Bluestein lines; out of place, in place and on strided
+    views, with and without a shift of every transformed axis on the output."""
+    import torch
+
+    from reikna_b200 import transformations as tr
+    from reikna_b200.fft import FFT
+
+    if shape[-1] == 256 and dtype == numpy.complex128:
+        pytest.skip("no plane pass of this size and type")
+    x = normal_array(rng, shape, dtype)
+    base = torch.zeros((2 * shape[0],) + shape[1:], dtype=torch.from_numpy(x).dtype, device=cuda)
+    t = base[1::2] if views else torch.empty(shape, dtype=base.dtype, device=cuda)
+    t.copy_(torch.from_numpy(x))
+    out = torch.empty_like(base)[::2] if views else torch.empty_like(t)
+    for inverse in (0, 1):
+        comp = FFT(t, axes=axes)
+        if shift:
+            sh = tr.fftshift(out, axes=axes)
+            comp.parameter.output.connect(sh, sh.input, shifted=sh.output)
+        call = comp.compile()
+        assert comp.describe(0)["passes"][0]["note"] == "plane" and call.launches == 3
+        call(None, out, t, inverse)
+        torch.cuda.synchronize()
+        ref = (numpy.fft.ifftn if inverse else numpy.fft.fftn)(x.astype(numpy.complex128), axes=axes)
+        if shift:
+            ref = numpy.fft.fftshift(ref, axes=axes)
+        bound = fft_bound(dtype, math.prod(shape[a] for a in axes))
+        assert rel_l2(out.cpu().numpy(), ref) < bound
+        same = t.clone() if not views else out
+        if views:
+            same.copy_(t)
+        call(None, same, same, inverse)
+        torch.cuda.synchronize()
+        assert rel_l2(same.cpu().numpy(), ref) < bound
+    assert torch.equal(t.cpu(), torch.from_numpy(x))
