@@ -45,8 +45,7 @@ struct MixPlan {
     uint32_t inplace;      // a thread has at most one butterfly a stage
     uint32_t bufs;         // buffers: one in place, or with nothing between first and last stage
     FastDiv r0;
-    MixStage stage[MIX_STAGES];   // (on 16 bytes: read as vectors)
-    FastDiv prdiv;         // by n / 2 + 1: bin pairs of a line (real transforms)
+    MixStage stage[MIX_STAGES];
 };
 
 // One side: a line index splits over the dims, innermost first; position j of the line is
@@ -84,6 +83,7 @@ struct LeanParams {
     // mixed-radix passes: the plan on the device, lines and threads a CTA, shared memory
     const MixPlan* mix;
     uint32_t mix_nl, mix_nt, mix_smem;
+    FastDiv mix_pairs;   // by n / 2 + 1, the bin pairs of a line (real transforms)
 };
 enum LeanReal : int32_t {
     LR_NYQ = 1,     // bin L is stored as well

@@ -257,71 +257,110 @@ __device__ __forceinline__ void mix_radix(const LeanParams& p, const MixPlan& x,
 #undef RK_MIX
 }
 
-// f(line, k) for the bin pairs k, n - k (k <= n / 2) of the tile's lines, one after another
-// over the CTA's threads.  Line by line, 26 of 384 threads had work at 50 samples: 41943 lines
-// of them, float32, RFFT 23.6 -> 6.6 us and IRFFT 26.5 -> 6.9, 116508 lines of 18 samples
-// 52.3 -> 7.1 and 63.5 -> 7.1.  (A tile of one line needs no division: with one, IRFFTs of 3000
-// to 12000 float64 samples took 3% longer.)
-template <class F> __device__ __forceinline__ void mix_pairs(const MixPlan& x, uint32_t lines, F f) {
-    const uint32_t pairs = x.prdiv.d;
-    if (x.nl == 1) {
-        for (uint32_t k = threadIdx.x; k < pairs; k += blockDim.x) f(0u, k);
-    } else {
-        for (uint32_t i = threadIdx.x; i < lines * pairs; i += blockDim.x) {
-            const uint32_t ln = fd_div(x.prdiv, i);
-            f(ln, i - ln * pairs);
+// A bin pair k, n - k (k <= n / 2) of a line of the tile
+template <typename V> struct MixPair {
+    const V* src;
+    V* dst;
+    uint32_t k;
+    V y[2];
+};
+
+// The bin pairs of the tile's lines, one after another over the CTA's threads, U of a thread
+// loaded before the first is used; line(ln) gives a line's pointers.  MANY: tiles of several lines.
+// Line by line, 26 of 384 threads had work at 50 samples: 41943 lines of them, float32, RFFT
+// 23.6 -> 6.6 us and IRFFT 26.5 -> 6.6, 116508 lines of 18 samples 52.3 -> 7.1 and 63.5 -> 7.0.
+template <bool MANY, int U, typename V, class Line, class Load, class Use>
+__device__ __forceinline__ void mix_pairs(const LeanParams& p, uint32_t lines, Line line, Load load, Use use) {
+    const uint32_t pairs = p.mix_pairs.d, total = MANY ? lines * pairs : pairs;
+    MixPair<V> q[U];
+    if constexpr (!MANY) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) line(q[u], 0u);
+    }
+    for (uint32_t i = threadIdx.x; i < total; i += U * blockDim.x) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t at = i + u * blockDim.x;
+            if (at < total) {
+                q[u].k = at;
+                if constexpr (MANY) {
+                    const uint32_t ln = fd_div(p.mix_pairs, at);
+                    line(q[u], ln);
+                    q[u].k = at - ln * pairs;
+                }
+                load(q[u]);
+            }
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i + u * blockDim.x < total) use(q[u]);
     }
 }
 
 // The real-spectrum step of the tile's lines: z (pitch and pads of the tile) to bins
 // X[0 .. n) and, where stored, X[n].  w_k = exp(-i pi k / n) in rmix.
-template <typename T>
+template <typename T, bool MANY>
 __device__ __forceinline__ void mix_bins_out(const LeanParams& p, const MixPlan& x, const cplx<T>* z, const uint32_t* off_st,
                                              uint32_t valid) {
     using V = cplx<T>;
     const V* wk = reinterpret_cast<const V*>(p.rmix);
     const uint32_t n = x.n;
     auto at = [&](uint32_t k) { return k + (x.pad ? fd_div(x.r0, k) : 0u); };
-    mix_pairs(x, valid, [&](uint32_t ln, uint32_t k) {
-        const V* zl = z + ln * x.pitch;
-        V* out = reinterpret_cast<V*>(p.st.base + off_st[ln]);
-        V o[2];
-        real_pair<T>(zl[at(k)], zl[at(k == 0 ? 0 : n - k)], __ldg(wk + k), T(0.5), o[0], o[1]);
-        if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
-        if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
-        out[k] = o[0];
-        if (k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * k < n) out[n - k] = o[1];
-    });
+    mix_pairs<MANY, 1, V>(
+        p, valid,
+        [&](MixPair<V>& q, uint32_t ln) {
+            q.src = z + ln * x.pitch;
+            q.dst = reinterpret_cast<V*>(p.st.base + off_st[ln]);
+        },
+        [&](MixPair<V>& q) {
+            q.y[0] = q.src[at(q.k)];
+            q.y[1] = q.src[at(q.k == 0 ? 0 : n - q.k)];
+        },
+        [&](MixPair<V>& q) {
+            V o[2];
+            real_pair<T>(q.y[0], q.y[1], __ldg(wk + q.k), T(0.5), o[0], o[1]);
+            if (p.st.flags & SF_PRE_CONJ) lean_conj<T, 2>(o);
+            if (p.st.flags & SF_SCALE) lean_scale<T, 2>(p.st, o);
+            q.dst[q.k] = o[0];
+            if (q.k == 0 ? (p.rflags & LR_NYQ) != 0 : 2 * q.k < n) q.dst[n - q.k] = o[1];
+        });
 }
 
 // The inverse step: bins of the tile's lines to the half-length spectrum, lines of n points.
-template <typename T>
+template <typename T, bool MANY>
 __device__ __forceinline__ void mix_bins_in(const LeanParams& p, const MixPlan& x, cplx<T>* z, const uint32_t* off_ld) {
     using V = cplx<T>;
     const V* wk = reinterpret_cast<const V*>(p.rmix);
     const uint32_t n = x.n;
-    mix_pairs(x, x.nl, [&](uint32_t ln, uint32_t k) {
-        const V* in = reinterpret_cast<const V*>(p.ld.base + off_ld[ln]);
-        V* zl = z + ln * n;
-        V y[2] = {in[k], in[n - k]}, a, b;
-        if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, y);
-        if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(y);
-        if (k == 0) {
-            // bins 0 and n of a real signal are real
-            y[0].y = T(0);
-            y[1].y = T(0);
-        }
-        real_pair<T>(y[0], y[1], __ldg(wk + k), T(0.5), a, b);
-        zl[k] = a;
-        if (k > 0 && 2 * k < n) zl[n - k] = b;
-    });
+    mix_pairs<MANY, 2, V>(
+        p, x.nl,
+        [&](MixPair<V>& q, uint32_t ln) {
+            q.src = reinterpret_cast<const V*>(p.ld.base + off_ld[ln]);
+            q.dst = z + ln * n;
+        },
+        [&](MixPair<V>& q) {
+            q.y[0] = q.src[q.k];
+            q.y[1] = q.src[n - q.k];
+        },
+        [&](MixPair<V>& q) {
+            V a, b;
+            if (p.ld.flags & SF_SCALE) lean_scale<T, 2>(p.ld, q.y);
+            if (p.ld.flags & SF_PRE_CONJ) lean_conj<T, 2>(q.y);
+            if (q.k == 0) {
+                // bins 0 and n of a real signal are real
+                q.y[0].y = T(0);
+                q.y[1].y = T(0);
+            }
+            real_pair<T>(q.y[0], q.y[1], __ldg(wk + q.k), T(0.5), a, b);
+            q.dst[q.k] = a;
+            if (q.k > 0 && 2 * q.k < n) q.dst[n - q.k] = b;
+        });
 }
 
 // REAL 1: the real-spectrum step after the FFT (RFFT: sample pairs in, bins out); 2: the
 // inverse step before it (IRFFT).  The mirror of bin k is bin n - k of the same line, both
 // in shared memory.
-template <typename T, int MODE, int REAL>
+template <typename T, int MODE, int REAL, bool MANY>
 __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(const __grid_constant__ LeanParams p) {
     using V = cplx<T>;
     extern __shared__ __align__(16) unsigned char rk_smem[];
@@ -344,7 +383,7 @@ __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(con
     __syncthreads();
     const uint32_t valid = min(x.nl, p.nlines - line0);
     if constexpr (REAL == 2) {
-        mix_bins_in<T>(p, x, buf0, off_ld);
+        mix_bins_in<T, MANY>(p, x, buf0, off_ld);
         __syncthreads();
         mix_radix<T, MODE, MIX_LINES, MIX_TILE>(p, x, 0, buf0, buf1, off_ld, off_st, valid);
         V* t = buf0;
@@ -371,7 +410,7 @@ __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(con
     if constexpr (REAL == 1) {
         mix_radix<T, MODE, MIX_TILE, MIX_LINES>(p, x, x.ns - 1, last, other, off_ld, off_st, valid);
         __syncthreads();
-        mix_bins_out<T>(p, x, other, off_st, valid);
+        mix_bins_out<T, MANY>(p, x, other, off_st, valid);
     } else {
         mix_radix<T, MODE, MIX_TILE, MIX_GLOBAL>(p, x, x.ns - 1, last, nullptr, off_ld, off_st, valid);
     }
@@ -379,10 +418,14 @@ __global__ void __launch_bounds__(MixCfg<T>::NT, MixCfg<T>::MINB) k_lean_mix(con
 
 template <typename T, int MODE, int REAL> struct LeanMixLauncher {
     static cudaError_t launch(const LeanParams& p, cudaStream_t st) {
-        return lean_launch(k_lean_mix<T, MODE, REAL>, (p.nlines + p.mix_nl - 1) / p.mix_nl, p.mix_nt, p.mix_smem, p, st);
+        return lean_launch(REAL && p.mix_nl > 1 ? k_lean_mix<T, MODE, REAL, (REAL > 0)> : k_lean_mix<T, MODE, REAL, false>,
+                           (p.nlines + p.mix_nl - 1) / p.mix_nl, p.mix_nt, p.mix_smem, p, st);
     }
     static cudaError_t prepare() {
-        return cudaFuncSetAttribute(k_lean_mix<T, MODE, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_lean_mix<T, MODE, REAL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
+        if (e != cudaSuccess || !REAL) return e;
+        return cudaFuncSetAttribute(k_lean_mix<T, MODE, REAL, (REAL > 0)>, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
     }
 };
 

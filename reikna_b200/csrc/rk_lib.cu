@@ -996,7 +996,7 @@ static int setup_lean(PassRec& r, const PassSpec& ps, int dbl, int64_t blue_n, c
     if (r.kind != PK_LINE || (r.var != 0 && r.var != 1 && r.var != 2)) return RK_OK;
     if (p.nlines >= (int64_t(1) << 31) || (p.ld.flags & SF_TW4)) return RK_OK;
     auto lp = std::make_shared<LeanPass>();
-    // up to four lines of 2^18 points (measured at LeanPick)
+    // up to four lines of 2^18 points, two of 2^19 (measured at LeanPick)
     const bool few = dbl && tw4 && !bvar && r.var == 0 && r.mode == MODE_LANE && r.L == 512 && p.nlines <= 2048;
     LeanParams& q = lp->prm;
     q = LeanParams{};
@@ -1108,8 +1108,11 @@ static int mix_radices(int64_t n, int* r) {
     int best = 1 << 30, nbest = 0, cur[MIX_STAGES];
     auto search = [&](auto&& self, int64_t left, int at, int top, int sum) -> void {
         if (left == 1) {
-            // (four stages with a 13 of an odd length stay with Bluestein: the plan notes of
-            // its two-CTA form are pinned at 4095 points)
+            // Four stages with a 13 of an odd length stay with Bluestein.  That is no faster (us,
+            // Bluestein against this form: 512 x 4095 complex64 25.2 and 16.4, 698 x 3003 30.2 and
+            // 16.5, 921 x 2275 complex128 107 and 30; of the forms timed only complex64 columns lose,
+            // 81 of 6435 points 20.2 and 31.1, 146 of 3575 17.8 and 18.8): the two-CTA form is held
+            // against the one-CTA form at 4095 points.
             const bool pinned = at > 3 && n % 2 && std::find(cur, cur + at, 13) != cur + at;
             if (at >= 2 && sum < best && !pinned) {
                 best = sum;
@@ -1139,8 +1142,9 @@ static int mix_radices(int64_t n, int* r) {
 // butterflies over the threads; the CTAs an SM holds (registers: 768 complex64 threads, 512
 // complex128; shared memory) share its issue slots, 25 R + 15 instructions a butterfly at
 // 2.45 a cycle; the tiles go in whole waves; strided lines pay for segments under 128 bytes.
-// The constants were fitted to 4400 timed (length, batch, tile) combinations: the tile it
-// takes is 3% slower than the best on average (60 to 6000 points, 2^18 to 2^21 elements).
+// The constants were fitted to 4400 timed (length, batch, tile) combinations of complex
+// transforms: the tile it takes is 3% slower than the best on average (60 to 6000 points, 2^18
+// to 2^21 elements).  The bin pairs of a real transform are not counted.
 static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int nsm, MixPlan& x, uint32_t* nt_out, uint32_t* smem_out) {
     int r[MIX_STAGES];
     const int ns = mix_radices(n, r);
@@ -1150,7 +1154,6 @@ static bool mix_tile(int64_t n, int dbl, int mode, int real, int64_t nlines, int
     x.ns = ns;
     x.pad = mode == MODE_POS && r[0] % 2 == 0;
     x.r0 = fast_div((uint32_t)r[0]);
-    x.prdiv = fast_div((uint32_t)(n / 2 + 1));
     x.pitch = (uint32_t)(n + (x.pad ? n / r[0] : 0));
     uint32_t P = 1, tw = 0;
     for (int s = 0; s < ns; ++s) {
@@ -1271,6 +1274,7 @@ template <class Alloc> static int setup_mix(PassRec& r, int dbl, int nsm, int or
     q.tw = tw;
     q.mix = (const MixPlan*)plan;
     q.mix_nl = x.nl;
+    q.mix_pairs = fast_div((uint32_t)(r.L / 2 + 1));
     q.nlines = (uint32_t)p.nlines;
     q.rev = order & 1;
     lp->only = true;
