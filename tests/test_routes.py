@@ -290,3 +290,19 @@ def test_planes_split_through_a_temporary(rng, cuda, dtype, shape, axes, shift, 
         torch.cuda.synchronize()
         assert rel_l2(same.cpu().numpy(), ref) < bound
     assert torch.equal(t.cpu(), torch.from_numpy(x))
+
+
+@pytest.mark.parametrize("form", ["rows", "columns"])
+def test_lengths_of_the_mixed_radix_tests_take_that_kernel(form):
+    """The lengths test_mixed_radix_lines runs are mixed-radix plans, but for odd ones of four
+    stages with a 13, and complex128 ones whose tile does not fit shared memory."""
+    from reikna_b200 import _native as N
+    from test_lean import MIXED
+
+    for fmt in (N.FMT_C64, N.FMT_C128):
+        for n in MIXED:
+            rows = 1 if n > 4000 else 3 if n > 700 else 67
+            shape, axis = ((rows, n), 1) if form == "rows" else ((2, n, 5 if n > 700 else 21), 1)
+            note = N.describe(N.desc(fmt, shape, (axis,)))["passes"][0]["note"]
+            expected = n not in (3003, 4095) and (fmt == N.FMT_C64 or n <= 6000)
+            assert (note == "mixed") == expected, (fmt, n, note)
