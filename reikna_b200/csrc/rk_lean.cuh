@@ -1,7 +1,7 @@
 // Lean line passes: a CTA transforms one tile of NL lines whose two sides are of the
-// pass' own complex type with plain strides and byte offsets that fit 32 bits (every
-// plan temporary, and user arrays below 4 GB without cropping off the axis, additive
-// terms or format conversions).  Others take line_body (rk_kernels.cuh).
+// pass' own complex type with plain strides and byte offsets that fit 32 bits (plan
+// temporaries and user arrays below 4 GB, the latter without cropping, additive terms or
+// format conversions).  Others take line_body (rk_kernels.cuh).
 //
 // What bounds them is HBM (16 or 32 bytes an element against a few dozen instructions),
 // as long as enough warps wait on loads at once, so they are built for occupancy and few
@@ -16,9 +16,9 @@
 // Measured on 16 Mi complex64 elements in three rotating buffer sets (a copy at the
 // measured peak takes 41.6 us): contiguous lines of 64 / 256 / 1024 / 4096 points 42.7 /
 // 43.1 / 44.9 / 49.2 us, strided ones of 32 / 128 / 256 / 512 points 43.2 / 47.0 / 49.2 /
-// 51.6 us.  Whole calls against the kernels that ran before: 16384 x 1024 inverse 61.7 ->
-// 46.4 us (persistent TMA-fed passes), 16 x 262144 84.9 -> 36.6 us (two strided passes with
-// table twiddles), 2048 x 2048 68.0 -> 39.1 us.
+// 51.6 us.  Whole calls against the kernels that ran before: 16384 x 1024 inverse 62.4 ->
+// 47.6 us (persistent TMA-fed passes), 16 x 262144 84.2 -> 32.5 us (two strided passes with
+// table twiddles), 2048 x 2048 67.4 -> 34.4 us.
 #pragma once
 #define RK_PACKED_F32   // packed complex64 sums (rk_dft.cuh)
 #include "rk_internal.h"
@@ -123,7 +123,8 @@ RK_LP(double, 1024, MODE_LANE, true, 16, 16, 4, 16)
 // Plan of a few complex128 lines' four-step first pass (VAR 8): 512-point columns on 8 elements
 // a thread, whose twice as many threads hide its chain of table twiddle loads while
 // they do not fill the GPU.  2^18 points, 8 against 16 elements: 1 line 14.7 us against 19.7, 2
-// 15.3 against 21.5, but 8 lines 48.6 against 46.9 and 64 328 against 285.
+// 15.3 against 21.5, 4 24.3 against 23.8, but 8 lines 48.6 against 46.9 and 64 328 against 285;
+// 2^19 points: 1 line 19.7 against 20.7, 2 30.9 both.
 template <typename T, int L, int MODE, int VAR> struct LeanPick {
     using P = LeanPlan<T, L, MODE, VAR == 1>;
 };

@@ -18,9 +18,9 @@
 // points for each line of N), so they hold 128 registers a thread at 32 elements (two
 // 256-thread CTAs an SM at M = 8192; the general kernel's paths took 255 and one CTA).
 // Measured, whole calls, against the general fused and four-pass kernels: 1000 x 3001
-// 86.0 -> 45.1 us, 1000 x 1000 over both axes 46.9 -> 28.7 us, 64 x 65521 281.9 -> 89.0 us
-// (columns 31 and 23 us, rows 40 us under ncu: issue slots 50% used, 15 to 21 of 64 warps
-// active, the rows' shared-memory and table reads 72% of the L1 data path).
+// 85.9 -> 42.7 us, 64 x 65521 279.4 -> 80.9 us (under ncu columns of 128 points 28 and 22 us,
+// rows of 1024 points 41 us: issue slots 53 to 54% used, 15 to 22 of 64 warps active, the L1
+// data path 49 to 55%).
 #pragma once
 #include "rk_lean.cuh"
 

@@ -10,8 +10,8 @@
 // itself at RT - j): one shuffle moves it, where lines live inside a warp.  The general
 // kernel wrote the whole line to shared memory and read it back between two block
 // barriers, at 64 registers with spills; what bounds both is instruction issue.
-// Measured, whole calls: spectrogram of 2^22 samples (1024 / 256) 41.1 -> 27.2 us, IRFFT of
-// 16384 x 513 bins 46.7 -> 29.0 us (a copy of its bytes 20.8 us), RFFT of 16384 x 1024 (pass
+// Measured, whole calls: spectrogram of 2^22 samples (1024 / 256) 41.0 -> 25.5 us, IRFFT of
+// 16384 x 513 bins 46.5 -> 27.9 us (a copy of its bytes 20.8 us), RFFT of 16384 x 1024 (pass
 // time) 41 -> 31 us, transposed spectrogram (pass time) 48 -> 37 us.
 #pragma once
 #include "rk_lean.cuh"
