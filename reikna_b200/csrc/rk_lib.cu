@@ -392,6 +392,7 @@ static int half_eligible(const rk_fft_desc& d, int dbl) {
 }
 
 static bool lean_allowed(const rk_fft_desc& d);
+static bool lean_load(const rk_fft_desc& d, const PassSpec& p);
 static bool plan_blue3(const rk_fft_desc& d, Planned& P, int ax, int64_t n, int64_t M, int64_t O, int64_t I, int cur, int out);
 static int plane_mid(const rk_fft_desc& d, const PassSpec& p);
 static bool mix_ok(const rk_fft_desc& d, const PassSpec& p);
@@ -554,6 +555,20 @@ static int plan_passes(const rk_fft_desc& d, Planned& P) {
                         // (wide segments of adjacent lines; 49.2 at 512, 53.4 at 1024)
                         N1 = int64_t(1) << (ilog2(n) / 2);
                         N2 = n / N1;
+                        // The general kernel's 128-point complex128 columns are slow on arrays L2
+                        // does not hold (float64 input, 64 x 256 against 128 x 128 points: 64 lines
+                        // 29.2 us against 26.7, but 128 lines 53.1 against 57.8 and 256 101 against 116;
+                        // complex128 on general kernels 23.2, 46.9, 81.5 against 21.6, 50.8, 89.2).
+                        if (dbl && N1 == 128 && N2 == 128 && O * n > (int64_t(1) << 20)) {
+                            PassSpec a;
+                            a.L = (int)N1; a.mode = MODE_LANE; a.axis = ax;
+                            a.O = O; a.C = N2;
+                            a.ld.buf = cur; a.ld.ax_len = n; a.ld.cA = 1; a.ld.jB = N2;
+                            if (!lean_load(d, a)) {
+                                N1 = 64;
+                                N2 = 256;
+                            }
+                        }
                     }
                     if (N1 > LM) { N1 = LM; N2 = n / N1; }
                     if (N2 > PM) {
@@ -1082,6 +1097,16 @@ static void pass_params(const rk_fft_desc& d, const PassSpec& ps, int dbl, PassP
     pp.nlines = ps.O * ps.C * ps.I;
     build_side(d, ps.ld, ps.axis, dbl, true, pp.ld);
     build_side(d, ps.st, ps.kind == PK_PLANE ? ps.axis2 : ps.axis, dbl, false, pp.st);
+}
+
+// Whether a lean body takes the load of a plain line pass.
+static bool lean_load(const rk_fft_desc& d, const PassSpec& p) {
+    const int dbl = d.dtype == RK_FMT_C128;
+    PassParams a;
+    LeanSide s;
+    if (!lean_allowed(d)) return false;
+    pass_params(d, p, dbl, a);
+    return lean_side(a.ld, a, dbl, p.L, p.mode == MODE_POS, 0, &s);
 }
 
 // Whether the load of `first` and the store of `last` (Bluestein passes over the axis'

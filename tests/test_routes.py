@@ -306,3 +306,33 @@ def test_lengths_of_the_mixed_radix_tests_take_that_kernel(form):
             note = N.describe(N.desc(fmt, shape, (axis,)))["passes"][0]["note"]
             expected = n not in (3003, 4095) and (fmt == N.FMT_C64 or n <= 6000)
             assert (note == "mixed") == expected, (fmt, n, note)
+
+
+@pytest.mark.parametrize("rows,real,flags,lengths", [(64, True, 0, [128, 128]), (65, True, 0, [64, 256]), (65, False, 0, [128, 128]),
+                                                     (65, False, 16, [64, 256]), (64, False, 16, [128, 128])])
+def test_long_complex128_lines_split_by_the_kernel_that_reads_them(rows, real, flags, lengths):
+    from reikna_b200 import _native as N
+
+    d = N.desc(N.FMT_C128, (rows, 2**14), (1,), flags)
+    if real:
+        d.input = N.edge(N.FMT_F64, (rows, 2**14))
+    assert [p["L"] for p in N.describe(d)["passes"]] == lengths
+
+
+@gpu
+def test_long_real_float64_lines_beyond_l2(cuda):
+    import torch
+
+    from reikna_b200 import _native as N
+
+    n = 2**14
+    d = N.desc(N.FMT_C128, (67, n), (1,))
+    d.input = N.edge(N.FMT_F64, (67, n))
+    torch.manual_seed(4)
+    x = torch.randn((67, n), dtype=torch.float64, device=cuda)
+    out = torch.empty((67, n), dtype=torch.complex128, device=cuda)
+    plan = N.Plan(d)
+    for inverse in (0, 1):
+        plan.execute([out.data_ptr()], [x.data_ptr()], inverse=inverse, stream=torch.cuda.current_stream().cuda_stream)
+        ref = (torch.fft.ifft if inverse else torch.fft.fft)(x, dim=1)
+        assert _rel(out, ref) < fft_bound(numpy.complex128, n)
