@@ -63,6 +63,7 @@ bool line_info(int dbl, int L, int mode, int var, LineInfo* out) {
         cudaError_t e_ = (call);                                                         \
         if (e_ != cudaSuccess) {                                                         \
             set_error(std::string(#call) + ": " + cudaGetErrorString(e_));               \
+            cudaGetLastError();   /* reported here, not by the next call */              \
             return e_ == cudaErrorMemoryAllocation ? RK_ERR_NOMEM : RK_ERR_CUDA;         \
         }                                                                                \
     } while (0)
@@ -1856,6 +1857,7 @@ int rk_fft_plan_create(const rk_fft_desc* desc, rk_fft_plan** out) {
         cudaError_t e = cudaMalloc(p, (size_t)std::max<int64_t>(bytes, 16));
         if (e != cudaSuccess) {
             set_error(std::string("temporary allocation failed: ") + cudaGetErrorString(e));
+            cudaGetLastError();
             return RK_ERR_NOMEM;
         }
         plan->temps.push_back(*p);
@@ -2330,6 +2332,7 @@ int build_call_params(rk_fft_plan* plan, void* const* outputs, int32_t n_outputs
             cudaThreadExchangeStreamCaptureMode(&mode);
             if (e != cudaSuccess) {
                 set_error("in-place staging allocation failed");
+                cudaGetLastError();
                 return RK_ERR_NOMEM;
             }
             plan->device_bytes += need;
@@ -2535,6 +2538,7 @@ int rk_fft_call(rk_fft_plan* plan, void* output, const void* input, int32_t inve
         const cudaError_t e = it.launch(q, (cudaStream_t)stream);
         if (e != cudaSuccess) {
             set_error(std::string("kernel launch failed: ") + cudaGetErrorString(e));
+            cudaGetLastError();   // (cudaLaunchKernelEx leaves it set for the next call)
             return RK_ERR_CUDA;
         }
     }
@@ -2580,6 +2584,7 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             e = pair_launch(r, p, prm[i + 1], p.status, st);
             if (e != cudaSuccess) {
                 set_error(std::string("kernel launch failed (pair): ") + cudaGetErrorString(e));
+                cudaGetLastError();
                 return RK_ERR_CUDA;
             }
             if (prof) {
@@ -2625,6 +2630,7 @@ int rk_fft_execute_user(rk_fft_plan* plan, void* const* outputs, int32_t n_outpu
             e = tma[i] ? r.ti.fn(p, r.nblocks, st) : r.li.fn(p, (p.nlines + r.li.nl - 1) / r.li.nl, st);
         if (e != cudaSuccess) {
             set_error(std::string("kernel launch failed (") + r.note + "): " + cudaGetErrorString(e));
+            cudaGetLastError();
             return RK_ERR_CUDA;
         }
         if (prof) CK(cudaEventRecord(plan->prof_ev[ev + 1], st));

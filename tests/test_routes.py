@@ -336,3 +336,51 @@ def test_long_real_float64_lines_beyond_l2(cuda):
         plan.execute([out.data_ptr()], [x.data_ptr()], inverse=inverse, stream=torch.cuda.current_stream().cuda_stream)
         ref = (torch.fft.ifft if inverse else torch.fft.fft)(x, dim=1)
         assert _rel(out, ref) < fft_bound(numpy.complex128, n)
+
+
+STALE = """
+import torch
+from reikna_b200 import _native as N
+x = torch.ones((4, 64), dtype=torch.complex64, device="cuda")
+out = torch.empty_like(x)
+lean, general = (N.Plan(N.desc(N.FMT_C64, (4, 64), (1,), f)) for f in (0, N.FLAG_NO_TMA))
+side = torch.cuda.Stream()
+torch.cuda.synchronize()
+refused = 0
+with torch.cuda.stream(side):
+    graph = torch.cuda.CUDAGraph()
+    graph.capture_begin(capture_error_mode="global")
+    try:
+        torch.cuda.synchronize()      # not permitted while a stream captures: ends the capture
+    except RuntimeError:
+        pass
+    for run in (lambda: lean.call(out.data_ptr(), x.data_ptr(), 0, side.cuda_stream),
+                lambda: lean.execute([out.data_ptr()], [x.data_ptr()], stream=side.cuda_stream)):
+        try:
+            run()
+        except N.NativeError:
+            refused += 1
+    try:
+        graph.capture_end()
+    except RuntimeError:
+        pass
+assert refused == 2
+out.zero_()
+stream = torch.cuda.current_stream().cuda_stream
+general.execute([out.data_ptr()], [x.data_ptr()], stream=stream)
+torch.cuda.synchronize()
+assert out[0, 0] == 64 and out[0, 1] == 0
+print("done")
+"""
+
+
+@gpu
+def test_a_refused_launch_leaves_no_error_behind(cuda):
+    """A launch the runtime refuses is that call's error, not the next call's."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parent.parent
+    res = subprocess.run([sys.executable, "-c", STALE], cwd=root, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and "done" in res.stdout, res.stdout + res.stderr
